@@ -63,7 +63,8 @@ struct State {
   int xw, xo1;       // x-face psi rows: width, first x of the high face's row
   long long plane;   // ny * pitch
   T db, dtm0, dte0dx, dx;
-  T rdx;   // 1 / dx correctly rounded (host IEEE division)
+  T rdx;         // 1 / dx correctly rounded (host IEEE division)
+  double rdx64;  // the same in double
   T prof[8][kMaxPml];
   // field sets: src is read, dst is written (the same set for the in-place
   // split kernels; ping-pong sets for the fused kernel)
@@ -167,31 +168,44 @@ struct InteriorBox {
   int chunks0, chunks;   // chunks of the first range, of both ranges
 };
 
-// Correctly rounded u / d for d > 0, given r = RN(1/d): Markstein's FMA
-// correction (P. W. Markstein, "Computation of elementary functions on the
-// IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1), 1990). With
-// r within half an ulp of 1/d and q0 = RN(u r) within one ulp of u/d, the
-// remainder u - d q0 is exact in one FMA and RN(q0 + r (u - d q0)) is the
-// correctly rounded quotient, as long as no step leaves the normal range.
-// |u| outside [2^-100, 2^100] (float; [2^-900, 2^900] double) takes the
-// IEEE division instead. Used for the CPML terms (c * dE) / dx, whose
-// divisor is the constant cell size.
-template <class T>
-__device__ __forceinline__ T div_const(T u, T d, T r) {
-  using M = R<T>;
-  const T lo = sizeof(T) == 4 ? T(7.8886090522101181e-31) : T(1.4708983551653345e-271);   // 2^-100, 2^-900
-  const T hi = sizeof(T) == 4 ? T(1.2676506002282294e+30) : T(6.7986211919640936e+270);   // 2^100, 2^900
-  const T a = u < T(0) ? -u : u;
+// Correctly rounded u / d for d > 0, given r = 1 / d correctly rounded in
+// double. Used for the CPML terms (c * dE) / dx, whose divisor is the
+// constant cell size.
+//
+// Floats: the double product u r is within 2^-52 of u / d, and the quotient
+// of two floats lies at least 2^-49 (relative) from every float rounding
+// boundary that it does not lie on; it lies on one only where d is a power of
+// two (the product is then exact) or, for a subnormal quotient, where
+// d >= 2. Its rounding to float is therefore the quotient's, for every u:
+// zeros keep their sign, infinities and NaN pass. Three instructions, no
+// range test and no branch, where Markstein's correction takes two products,
+// two FMAs, a range test and a branch per term, and below 2^-100, which the
+// faint front of a wave meets, the IEEE division. Measured: a 32-member
+// batch 1.35 ms per step with the correction, 1.31 so.
+__device__ __forceinline__ float div_const(float u, float, double r) {
+  return __double2float_rn(__dmul_rn((double)u, r));
+}
+
+// Doubles: Markstein's FMA correction (P. W. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Develop. 34(1), 1990). With r within half an ulp of 1/d and q0 = RN(u r)
+// within one ulp of u/d, the remainder u - d q0 is exact in one FMA and
+// RN(q0 + r (u - d q0)) is the correctly rounded quotient, as long as no step
+// leaves the normal range. |u| outside [2^-900, 2^900] takes the IEEE
+// division instead.
+__device__ __forceinline__ double div_const(double u, double d, double r) {
+  const double lo = 1.4708983551653345e-271, hi = 6.7986211919640936e+270;   // 2^-900, 2^900
+  const double a = fabs(u);
   if (a >= lo && a <= hi) {
-    const T q0 = M::mul(u, r);
-    const T rem = M::fma(-q0, d, u);
-    return M::fma(rem, r, q0);
+    const double q0 = __dmul_rn(u, r);
+    const double rem = __fma_rn(-q0, d, u);
+    return __fma_rn(rem, r, q0);
   }
-  return a == T(0) ? u : M::div(u, d);   // zeros keep their sign; tiny, huge, NaN: IEEE
+  return a == 0.0 ? u : __ddiv_rn(u, d);   // zeros keep their sign; tiny, huge, NaN: IEEE
 }
 
 template <class T>
-__device__ __forceinline__ T div_dx(const State<T>& s, T u) { return div_const(u, s.dx, s.rdx); }
+__device__ __forceinline__ T div_dx(const State<T>& s, T u) { return div_const(u, s.dx, s.rdx64); }
 
 // Index of cell x of plane z, row y in an x-face psi array of side `side`.
 template <class T>

@@ -1,7 +1,7 @@
 // fdtd_selfcheck.cu -- device check of the division by the cell size.
 //
-// The CPML terms divide by the constant cell size with Markstein's FMA
-// correction (div_const, fdtd_common.cuh) instead of an IEEE division. This
+// The CPML terms divide by the constant cell size through its reciprocal
+// (div_const, fdtd_common.cuh) instead of an IEEE division. This
 // entry point runs both on the device and counts the inputs whose results
 // differ in any bit: every one of the 2^32 float bit patterns, or 2^30
 // doubles (random significands over the exponents where the correction is
@@ -22,7 +22,7 @@ __device__ __forceinline__ bool same_bits_d(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b) || (a != a && b != b);
 }
 
-__global__ void k_check_div_f(float d, float r, unsigned long long* bad) {
+__global__ void k_check_div_f(float d, double r, unsigned long long* bad) {
   unsigned long long local = 0;
   const unsigned long long n = 1ULL << 32;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -81,7 +81,7 @@ extern "C" int fdtd_check_cell_division(int dtype, double cell_size, int device,
   unsigned long long n;
   if (dtype == FDTD_F32) {
     const float d = (float)cell_size;
-    const float r = 1.0f / d;   // IEEE division on the host
+    const double r = 1.0 / (double)d;   // IEEE division on the host
     n = 1ULL << 32;
     k_check_div_f<<<148 * 16, 256>>>(d, r, bad);
   } else {

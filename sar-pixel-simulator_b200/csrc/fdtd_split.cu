@@ -110,10 +110,12 @@ __device__ __forceinline__ const ShellBox& find_box(const ShellBoxes& bl, int bi
   return bl.b[k];
 }
 
-// Resident blocks per SM the split passes ask for (float: register cap 64;
-// the passes are latency-bound, so more warps in flight beat a few spills)
+// Resident blocks per SM the split passes ask for (float: register cap 72;
+// the passes are latency-bound, but at 64 registers the division's double
+// products spill: a 32-member batch takes 1.40 ms per step with 8 blocks,
+// 1.31 with 7)
 template <class T>
-constexpr int split_min_blocks() { return sizeof(T) == 4 ? 8 : 1; }
+constexpr int split_min_blocks() { return sizeof(T) == 4 ? 7 : 1; }
 
 template <class T, bool kH>
 __global__ void __launch_bounds__(128, split_min_blocks<T>()) k_shell(State<T> s, const int* __restrict__ tp, int toff,
@@ -498,9 +500,9 @@ void launch_shell_pass(const State<T>& s, const int* tdev, int toff, const Shell
   if (bl.n == 0 || bl.total_blocks == 0) return;
   // Several planes per block amortise the block's set-up, but only where
   // one plane per block gives many waves of blocks: 148 SMs hold about
-  // 1184 of these blocks at once (8 each). add_shell_box numbered the
+  // 1036 of these blocks at once (7 each). add_shell_box numbered the
   // blocks one plane each; renumber for the choice.
-  constexpr int kResident = 148 * 8;
+  constexpr int kResident = 148 * 7;
   ShellBoxes p = bl;
   p.planes = bl.total_blocks >= 16 * kResident ? 4 : bl.total_blocks >= 8 * kResident ? 2 : 1;
   p.total_blocks = 0;
