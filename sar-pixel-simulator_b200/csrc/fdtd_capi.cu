@@ -1215,22 +1215,6 @@ extern "C" int fdtd_near2far(const void* ex_u, const void* ey_u, const void* hx_
   if (device < 0 || device >= ndev) return fail(FDTD_ERR_INVALID, "device %d out of range", device);
   DeviceGuard device_guard;   // the caller's current device is restored on return
   CK(cudaSetDevice(device));
-  // surface currents in complex128, as near2far.py:64-68 converts them:
-  // Jx = -Hy, Jy = Hx, Mx = Ey, My = -Ex   (near2far.py:94-96)
-  const size_t n = (size_t)nx_ph * ny_ph;
-  std::vector<double> jm(8 * n);
-  auto get = [&](const void* p, size_t i, int part) -> double {
-    return in_dtype == FDTD_F32 ? (double)((const float*)p)[2 * i + part]
-                                : ((const double*)p)[2 * i + part];
-  };
-  for (size_t i = 0; i < n; ++i) {
-    for (int part = 0; part < 2; ++part) {
-      jm[2 * (0 * n + i) + part] = -get(hy_u, i, part);
-      jm[2 * (1 * n + i) + part] = get(hx_u, i, part);
-      jm[2 * (2 * n + i) + part] = get(ey_u, i, part);
-      jm[2 * (3 * n + i) + part] = -get(ex_u, i, part);
-    }
-  }
   std::vector<double> th(ntheta), ph(nphi);
   for (int i = 0; i < ntheta; ++i) th[i] = thetas_deg[i] * (M_PI / 180.0);
   for (int i = 0; i < nphi; ++i) ph[i] = phis_deg[i] * (M_PI / 180.0);
@@ -1238,32 +1222,36 @@ extern "C" int fdtd_near2far(const void* ex_u, const void* ey_u, const void* hx_
   const double lam = c0 / freq;
   const double k = 2.0 * M_PI / lam;
   const double z_val = (double)((nz_ph - 1) / 2) * dx;
-  double *djm = nullptr, *dth = nullptr, *dph = nullptr, *dout = nullptr;
-  const size_t out_n = (size_t)8 * nphi * ntheta;
+  const size_t pb = (size_t)nx_ph * ny_ph * (in_dtype == FDTD_F32 ? 8 : 16);
+  const size_t ab = sizeof(double) * (size_t)(ntheta + nphi), ob = sizeof(double) * (size_t)8 * nphi * ntheta;
+  const long long angles = (long long)nphi * ntheta;
+  const size_t sb = near2far_scratch(nx_ph, ny_ph, (int)std::min<long long>(angles, INT32_MAX));
+  // one allocation: the planes as given, scratch, output, angles
+  auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+  th.insert(th.end(), ph.begin(), ph.end());
+  unsigned char* d = nullptr;
   cudaStream_t st;
   CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   int rc = FDTD_OK;
   do {
-    if (cudaMallocAsync(&djm, jm.size() * sizeof(double), st) != cudaSuccess ||
-        cudaMallocAsync(&dth, th.size() * sizeof(double), st) != cudaSuccess ||
-        cudaMallocAsync(&dph, ph.size() * sizeof(double), st) != cudaSuccess ||
-        cudaMallocAsync(&dout, out_n * sizeof(double), st) != cudaSuccess) {
+    if (cudaMallocAsync((void**)&d, up(4 * pb) + up(sb) + up(ob) + up(ab), st) != cudaSuccess) {
       rc = fail(FDTD_ERR_NOMEM, "near2far device allocation failed");
       break;
     }
-    cudaMemcpyAsync(djm, jm.data(), jm.size() * sizeof(double), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(dth, th.data(), th.size() * sizeof(double), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(dph, ph.data(), ph.size() * sizeof(double), cudaMemcpyHostToDevice, st);
-    if (near2far_run(djm, nx_ph, ny_ph, dx, z_val, k, dth, ntheta, dph, nphi, r, dout, st)) {
+    unsigned char* const scratch = d + up(4 * pb);
+    double* const dout = (double*)(scratch + up(sb));
+    double* const dth = (double*)((unsigned char*)dout + up(ob));
+    cudaMemcpyAsync(dth, th.data(), ab, cudaMemcpyHostToDevice, st);
+    const void* planes[4] = {ex_u, ey_u, hx_u, hy_u};
+    for (int c = 0; c < 4; ++c) cudaMemcpyAsync(d + c * pb, planes[c], pb, cudaMemcpyHostToDevice, st);
+    if (near2far_run(d, in_dtype == FDTD_F32, nx_ph, ny_ph, dx, z_val, k, dth, ntheta, dth + ntheta, nphi, r, scratch,
+                     dout, st)) {
       rc = fail(FDTD_ERR_CUDA, "near2far launch failed: %s", cudaGetErrorString(cudaGetLastError()));
       break;
     }
-    cudaMemcpyAsync(out, dout, out_n * sizeof(double), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(out, dout, ob, cudaMemcpyDeviceToHost, st);
   } while (0);
-  if (djm) cudaFreeAsync(djm, st);
-  if (dth) cudaFreeAsync(dth, st);
-  if (dph) cudaFreeAsync(dph, st);
-  if (dout) cudaFreeAsync(dout, st);
+  if (d) cudaFreeAsync(d, st);
   cudaError_t e = cudaStreamSynchronize(st);
   cudaStreamDestroy(st);
   if (rc == FDTD_OK && e != cudaSuccess)

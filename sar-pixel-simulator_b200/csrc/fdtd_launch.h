@@ -242,9 +242,13 @@ void launch_paint_spheres(T* eps, T* sig, int nx, int ny, int nz_mat, const doub
 // Records an error message for fdtd_last_error(); returns code.
 int report_error(int code, const char* msg);
 
-// Near-to-far transform (near2far.cu).
-int near2far_run(const double* jm /* 4 planes complex128 */, int nx, int ny, double dx,
-                 double z_val, double k, const double* thetas, int ntheta,
-                 const double* phis, int nphi, double r, double* out, cudaStream_t st);
+// Near-to-far transform (near2far.cu) of the planes ex, ey, hx, hy as given
+// (complex64 with `single`, else complex128; device, one after another) into
+// out (4 x (nphi, ntheta) complex128, device); angles in radians (device).
+// scratch: near2far_scratch bytes. Returns 0 or 1 (CUDA error).
+size_t near2far_scratch(int nx, int ny, int angles);
+int near2far_run(const void* planes, bool single, int nx, int ny, double dx, double z_val, double k,
+                 const double* thetas, int ntheta, const double* phis, int nphi, double r, void* scratch, double* out,
+                 cudaStream_t st);
 
 }  // namespace fdtd
