@@ -800,6 +800,31 @@ static int upload_volume(fdtd_sim* s, void* dst, const void* src) {
   return FDTD_OK;
 }
 
+// `rows` pitched device rows to packed host rows: packed on the device in
+// pieces that fit the handle's packed buffer, each piece one contiguous
+// transfer (a pitched copy when the buffer cannot be had). Enqueued on the
+// handle's stream.
+static int download_rows(fdtd_sim* s, void* dst, const void* src, long long rows) {
+  const size_t w = (size_t)s->g.nx * s->esz;
+  const long long room = (long long)s->g.ny * s->g.nz;
+  if (!s->packed && alloc(s, w * room, &s->packed) != FDTD_OK) s->packed = nullptr;
+  if (!s->packed) {
+    CK(cudaMemcpy2DAsync(dst, w, src, (size_t)s->pitch * s->esz, w, (size_t)rows, cudaMemcpyDeviceToHost, s->stream));
+    return FDTD_OK;
+  }
+  s->mat_nz = -1;   // a staged material block is gone
+  for (long long r = 0; r < rows; r += room) {
+    const long long n = std::min(room, rows - r);
+    if (s->g.dtype == FDTD_F32)
+      launch_unpitch<float>((float*)s->packed, (const float*)src + r * s->pitch, s->g.nx, n, s->pitch, s->stream);
+    else
+      launch_unpitch<double>((double*)s->packed, (const double*)src + r * s->pitch, s->g.nx, n, s->pitch, s->stream);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync((unsigned char*)dst + r * w, s->packed, w * n, cudaMemcpyDeviceToHost, s->stream));
+  }
+  return FDTD_OK;
+}
+
 int fdtd_set_materials(fdtd_sim* s, const void* ca, const void* cb) {
   DeviceGuard device_guard;   // the caller's current device is restored on return
   int rc = check_sim(s);
@@ -2245,12 +2270,9 @@ int fdtd_incident_get_planes(fdtd_incident* b, void* ex, void* ey, void* hx, voi
   if (rc) return rc;
   if (!b->ran) return fail(FDTD_ERR_STATE, "incident run not done (fdtd_incident_run)");
   fdtd_sim* s = b->sim;
-  const size_t w = (size_t)s->g.nx * s->esz;
   void* dst[4] = {ex, ey, hx, hy};
   for (int c = 0; c < 4; ++c)
-    if (dst[c])
-      CK(cudaMemcpy2DAsync(dst[c], w, b->rec[c], (size_t)s->pitch * s->esz, w, (size_t)s->g.ny * s->g.nt,
-                           cudaMemcpyDeviceToHost, s->stream));
+    if (dst[c] && (rc = download_rows(s, dst[c], b->rec[c], (long long)s->g.ny * s->g.nt))) return rc;
   CK(cudaStreamSynchronize(s->stream));
   return FDTD_OK;
 }

@@ -90,6 +90,9 @@ void launch_batch_shell(const BatchModel<T>* bm, const BatchShellBox* boxes, int
 // Packed rows of nx elements into rows of `pitch` elements.
 template <class T>
 void launch_repitch(T* dst, const T* src, int nx, long long rows, int pitch, cudaStream_t st);
+// Rows of `pitch` elements into packed rows of nx.
+template <class T>
+void launch_unpitch(T* dst, const T* src, int nx, long long rows, int pitch, cudaStream_t st);
 
 template <class T>
 void launch_eps_sigma(int nx, int ny, int nz, int nz_mat, int pitch, const T* eps,

@@ -563,6 +563,25 @@ void launch_repitch(T* dst, const T* src, int nx, long long rows, int pitch, cud
   k_repitch<T><<<grd, 256, 0, st>>>(dst, src, nx, rows, pitch);
 }
 
+// Pitched rows into packed ones, for read-backs: a pitched device-to-host
+// copy of short rows moves one row at a time (133-cell rows into pageable
+// memory: 17 ms for 34 MB).
+template <class T>
+__global__ void __launch_bounds__(256) k_unpitch(T* __restrict__ dst, const T* __restrict__ src, int nx,
+                                                 long long rows, int pitch) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= nx) return;
+  for (long long r = blockIdx.y; r < rows; r += gridDim.y) dst[r * nx + x] = src[r * pitch + x];
+}
+
+template <class T>
+void launch_unpitch(T* dst, const T* src, int nx, long long rows, int pitch, cudaStream_t st) {
+  const dim3 grd((nx + 255) / 256, (unsigned)std::min<long long>(rows, 65535), 1);
+  k_unpitch<T><<<grd, 256, 0, st>>>(dst, src, nx, rows, pitch);
+}
+
+template void launch_unpitch<float>(float*, const float*, int, long long, int, cudaStream_t);
+template void launch_unpitch<double>(double*, const double*, int, long long, int, cudaStream_t);
 template void launch_repitch<float>(float*, const float*, int, long long, int, cudaStream_t);
 template void launch_repitch<double>(double*, const double*, int, long long, int, cudaStream_t);
 
