@@ -79,6 +79,17 @@ extern "C" {
 #define FDTD_OPT_SHELL        11 /* how the fused step updates the shell around
                                     its interior box: FDTD_SHELL_* */
 #define FDTD_OPT_BATCH_MODE   12 /* fdtd_batch_set_option: FDTD_BATCH_* */
+#define FDTD_OPT_MULTISTEP    13 /* FDTD_MULTI_*: FDTD_KERNEL_FUSED may
+                                    advance several steps per launch, with the
+                                    same results bit for bit (default 0). Not
+                                    used while FDTD_OPT_CHECK_EVERY is on */
+
+/* several steps per launch (fdtd_set_option(FDTD_OPT_MULTISTEP, ...)) */
+#define FDTD_MULTI_OFF      0
+#define FDTD_MULTI_AUTO     1 /* by the grid's size: pair or single */
+#define FDTD_MULTI_PAIR     3 /* two steps per pass over the fields; holds a
+                                 third field set (single steps where there is
+                                 no memory for it, or the grid is too narrow) */
 
 /* batched sweep (fdtd_batch_set_option(FDTD_OPT_BATCH_MODE, ...)) */
 #define FDTD_BATCH_SPLIT   0   /* (default) one launch per pass (H, E, phasors)

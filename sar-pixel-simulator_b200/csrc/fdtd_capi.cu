@@ -76,7 +76,8 @@ struct fdtd_sim {
   long long ph_off[24];
   long long ph_elems = 0;
   double* phase = nullptr;
-  int* tdev = nullptr;
+  int* tdev = nullptr;                   // step counter; [2] stays 0;
+                                         // [6] set by a kernel when a wait inside it ran out
   int* flags = nullptr;                  // non-finite check: found, step
   int64_t t = 0;
   int cur = 0;
@@ -122,11 +123,23 @@ struct fdtd_sim {
   int plan_ok = 0, plan_tile_y = 0, plan_zchunk = 0, plan_slab = 0, plan_shell = 0;
   int graph_chunk = 0;
   int check_every = 0;
+  // FDTD_OPT_MULTISTEP: the pair step (0 not looked at, 1 ready, -1 not for
+  // this grid or no memory for it), its plan and tensor maps (one set per
+  // source set), a third stream for its z-face chunks
+  int multi = 0;
+  int pair_state = 0;
+  PairPlan pair;
+  PairMapSet pmaps[2];
+  void* pair_mid = nullptr;              // the planes of a PairMid
+  cudaStream_t side2 = nullptr;
+  cudaEvent_t join2 = nullptr;
+  bool wait_look = false;                // such kernels were enqueued since the last look
   // captured step chunks (FDTD_OPT_GRAPH_CHUNK), one per starting field set,
   // with the settings they were captured under; absorber uploads bump the
   // epoch (the profiles are captured by value)
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  int gsig[2][9] = {};
+  int gsig[2][10] = {};
+  int gend[2] = {};                      // the current set after a replay
   int graph_epoch = 0;
   // gradient (fdtd_grad_*): checkpoints of the forward solve, the segment
   // of recomputed states and the adjoint state; a state is the 6 fields
@@ -143,7 +156,8 @@ struct fdtd_sim {
   double* grad_gim = nullptr;
   // per-kernel event timing
   int timing = 0;
-  std::vector<cudaEvent_t> ev;   // 3 per timed step: before step, after step, after phasors
+  std::vector<cudaEvent_t> ev;   // 3 per timed launch group: before step, after step, after phasors
+  std::vector<int> ev_steps;     // steps of each group
   int ev_used = 0;
   double acc_ms[2] = {0, 0};
   int acc_n[2] = {0, 0};
@@ -216,6 +230,18 @@ int take_bounds_violation() {
                 (long long)what, line);
   return fail(FDTD_ERR_BOUNDS, "bounds check: %llu bad accesses; the first: %lld bytes at address 0x%llx (line %lld)",
               n, bytes, what, line);
+}
+
+// A wait inside a kernel that ran out since the last look (the results of
+// that run are not valid). After a synchronisation of the handle's stream.
+int take_wait_error(fdtd_sim* s) {
+  if (!s->wait_look) return FDTD_OK;
+  s->wait_look = false;
+  int w = 0;
+  CK(cudaMemcpy(&w, s->tdev + 6, sizeof(w), cudaMemcpyDeviceToHost));
+  if (!w) return FDTD_OK;
+  CK(cudaMemset(s->tdev + 6, 0, sizeof(w)));
+  return fail(FDTD_ERR_CUDA, "a wait inside a step kernel ran out: the run's results are not valid");
 }
 
 void release(fdtd_sim* s, void* p) {
@@ -339,15 +365,101 @@ int collect_timing(fdtd_sim* s) {
     float a = 0, b = 0;
     CK(cudaEventElapsedTime(&a, s->ev[i], s->ev[i + 1]));
     CK(cudaEventElapsedTime(&b, s->ev[i + 1], s->ev[i + 2]));
-    s->acc_ms[0] += a; s->acc_n[0] += 1;
-    s->acc_ms[1] += b; s->acc_n[1] += 1;
+    const int n = s->ev_steps[i / 3];
+    s->acc_ms[0] += a; s->acc_n[0] += n;
+    s->acc_ms[1] += b; s->acc_n[1] += n;
   }
   s->ev_used = 0;
+  s->ev_steps.clear();
+  return FDTD_OK;
+}
+
+// What the pair step needs beyond two field sets, made on first use: the
+// mid planes, the plan and maps. A grid without a column worth marching, or
+// a device without room, takes single steps.
+template <class T>
+bool pair_ready(fdtd_sim* s) {
+  if (s->pair_state) return s->pair_state > 0;
+  s->pair_state = -1;
+  const fdtd_geometry& g = s->g;
+  s->pair = make_pair_plan(g.nx, g.ny, g.nz, g.npml, (int)sizeof(T));
+  if (!s->pair.ok) return false;
+  const std::string msg = g_err;   // running in single steps is no error
+  long long n[3];
+  pair_mid_sizes<T>(make_state<T>(s, 0, 0), n);
+  bool ok = alloc(s, (size_t)(4 * n[0] + 4 * n[1] + 8 * n[2]) * sizeof(T), &s->pair_mid) == FDTD_OK;
+  for (int k = 0; k < 2 && ok; ++k) ok = make_pair_maps<T>(make_state<T>(s, k, 1 - k), &s->pmaps[k]);
+  ok = ok && (s->side2 || cudaStreamCreateWithFlags(&s->side2, cudaStreamNonBlocking) == cudaSuccess);
+  ok = ok && (s->join2 || cudaEventCreateWithFlags(&s->join2, cudaEventDisableTiming) == cudaSuccess);
+  if (!ok) {
+    release(s, s->pair_mid);
+    s->pair_mid = nullptr;
+    cudaGetLastError();
+    g_err = msg;
+    return false;
+  }
+  s->pair_state = 1;
+  return true;
+}
+
+// Steps k and k + 1 of the run in one pass: the marches of the four kinds
+// of regions read the source set and write disjoint cells of the
+// destination set, side by side on three streams.
+template <class T>
+int enqueue_pair(fdtd_sim* s, int k, int ph_g0, int ph_ng, cudaEvent_t after_step) {
+  const int nxt = 1 - s->cur;
+  const State<T> st = make_state<T>(s, s->cur, nxt);
+  PairMid<T> mid;
+  {
+    long long sizes[3];
+    pair_mid_sizes<T>(st, sizes);
+    T* q = (T*)s->pair_mid;
+    for (int c = 0; c < 4; ++c, q += sizes[0]) mid.z[c] = q;
+    for (int c = 0; c < 4; ++c, q += sizes[1]) mid.y[c] = q;
+    for (int t = 0; t < 2; ++t)
+      for (int c = 0; c < 4; ++c, q += sizes[2]) mid.x[t][c] = q;
+  }
+  CK(cudaEventRecord(s->fork, s->stream));
+  CK(cudaStreamWaitEvent(s->side, s->fork, 0));
+  CK(cudaStreamWaitEvent(s->side2, s->fork, 0));
+  const PairMapSet& maps = s->pmaps[s->cur];
+  s->wait_look = true;
+  if (!launch_pair<T>(kPairX, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side) ||
+      !launch_pair<T>(kPairY, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side2) ||
+      !launch_pair<T>(kPairPlain, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->stream) ||
+      !launch_pair<T>(kPairZ, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side2))
+    return fail(FDTD_ERR_CUDA, "pair step launch: %s", cudaGetErrorString(cudaGetLastError()));
+  CK(cudaEventRecord(s->join, s->side));
+  CK(cudaEventRecord(s->join2, s->side2));
+  CK(cudaStreamWaitEvent(s->stream, s->join, 0));
+  CK(cudaStreamWaitEvent(s->stream, s->join2, 0));
+  s->cur = nxt;
+  mark(s, after_step);
+  launch_phasors_pair<T>(make_state<T>(s, nxt, nxt), mid, s->tdev, k, s->stream, ph_g0, ph_ng);
   return FDTD_OK;
 }
 
 // ph_g0, ph_ng: the phasor plane groups each step accumulates (all six by
 // default; none with ph_ng = 0; the gradient's forward only the upper plane)
+// The path of a run of n steps. FDTD_MULTI_AUTO takes the fastest on the B200
+// (us per step; single, pair):
+//   float  0.97 M cells  49  57      double  0.97 M   84   71
+//          4.32 M       104  91              1.78 M  119   92
+//          14.7 M       230 186              14.7 M  635  328
+// The pair step wins once the plain box outweighs its ends: in float also
+// only on wide grids (91 x 267 x 133 cells: 92 single, 104 pair;
+// 301 x 121 x 121: 116 and 135; 61 x 401 x 201: 125 and 111).
+constexpr long long kPairCellsFloat = 4000000, kPairCellsDouble = 1500000;
+constexpr int kPairNxFloat = 160;
+
+bool takes_pair(const fdtd_sim* s) {
+  if (s->kernel != FDTD_KERNEL_FUSED || s->check_every > 0) return false;
+  if (s->multi == FDTD_MULTI_PAIR) return true;
+  const long long cells = (long long)s->g.nx * s->g.ny * s->g.nz;
+  return s->multi == FDTD_MULTI_AUTO &&
+         (s->esz == 8 ? cells >= kPairCellsDouble : cells >= kPairCellsFloat && s->g.nx >= kPairNxFloat);
+}
+
 template <class T>
 int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
   for (int k = 0; k < n; ++k) {
@@ -358,7 +470,18 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     cudaEvent_t e0 = s->timing ? timing_event(s) : nullptr;
     cudaEvent_t e1 = s->timing ? timing_event(s) : nullptr;
     cudaEvent_t e2 = s->timing ? timing_event(s) : nullptr;
+    if (s->timing) s->ev_steps.push_back(1);
     mark(s, e0);
+    // FDTD_OPT_MULTISTEP: two steps per pass, unless the fields are to be
+    // looked at after every step
+    if (takes_pair(s) && k + 2 <= n && pair_ready<T>(s)) {
+      const int rc = enqueue_pair<T>(s, k, ph_g0, ph_ng, e1);
+      if (rc) return rc;
+      mark(s, e2);
+      if (s->timing) s->ev_steps.back() = 2;
+      ++k;
+      continue;
+    }
     if (s->kernel == FDTD_KERNEL_FUSED) {
       const int nxt = 1 - s->cur;
       if (!fused_supported_tile(s->tile_x, s->tile_y, (int)sizeof(T)))
@@ -431,8 +554,9 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
 template <class T>
 int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
   const int start = s->cur;
-  const int sig[9] = {chunk,          s->kernel,      s->tile_x,    s->tile_y, s->zchunk,
-                      s->phasor_mode, s->graph_epoch, s->slab, s->shell};
+  if (takes_pair(s)) pair_ready<T>(s);   // allocates: not during a capture
+  const int sig[10] = {chunk,          s->kernel,      s->tile_x, s->tile_y, s->zchunk,
+                       s->phasor_mode, s->graph_epoch, s->slab,   s->shell,  s->multi};
   if (!s->gexec[start] || memcmp(sig, s->gsig[start], sizeof(sig)) != 0) {
     if (s->gexec[start]) {
       cudaGraphExecDestroy(s->gexec[start]);
@@ -442,6 +566,7 @@ int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
     const int rc = enqueue_steps<T>(s, chunk);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
+    s->gend[start] = s->cur;
     s->cur = start;   // capturing ran nothing
     if (rc || e != cudaSuccess) {
       if (graph) cudaGraphDestroy(graph);
@@ -457,7 +582,8 @@ int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
     memcpy(s->gsig[start], sig, sizeof(sig));
   }
   CK(cudaGraphLaunch(s->gexec[start], s->stream));
-  if (s->kernel == FDTD_KERNEL_FUSED && (chunk & 1)) s->cur = 1 - start;
+  s->wait_look = s->wait_look || s->multi != FDTD_MULTI_OFF;
+  s->cur = s->gend[start];
   return FDTD_OK;
 }
 
@@ -614,7 +740,7 @@ int fdtd_create(const fdtd_geometry* geom, int device, fdtd_sim** out) {
   A((size_t)off * s->esz, &s->ph);
   A((size_t)off * s->esz, &s->phc);
   A((size_t)std::max(g.nt, 1) * 4 * sizeof(double), (void**)&s->phase);
-  A(sizeof(int) * 4, (void**)&s->tdev);
+  A(sizeof(int) * 8, (void**)&s->tdev);
   A(sizeof(int) * 2, (void**)&s->flags);
   if (rc != FDTD_OK) {
     fdtd_destroy(s);
@@ -677,6 +803,7 @@ int fdtd_destroy(fdtd_sim* s) {
     cudaFree(b.p);
   }
   if (s->side) cudaStreamSynchronize(s->side);
+  if (s->side2) cudaStreamSynchronize(s->side2);
   if (s->copy) cudaStreamSynchronize(s->copy);
   for (int k = 0; k < 2; ++k) {
     if (s->copy_ev[k]) cudaEventDestroy(s->copy_ev[k]);
@@ -689,6 +816,8 @@ int fdtd_destroy(fdtd_sim* s) {
   if (s->fork) cudaEventDestroy(s->fork);
   if (s->join) cudaEventDestroy(s->join);
   if (s->side) cudaStreamDestroy(s->side);
+  if (s->join2) cudaEventDestroy(s->join2);
+  if (s->side2) cudaStreamDestroy(s->side2);
   if (s->own) cudaStreamDestroy(s->own);
   delete s;
   cudaGetLastError();
@@ -742,6 +871,11 @@ int fdtd_set_option(fdtd_sim* s, int option, int value) {
     case FDTD_OPT_TIMING:
       s->timing = value ? 1 : 0;
       return FDTD_OK;
+    case FDTD_OPT_MULTISTEP:
+      if (value < FDTD_MULTI_OFF || value > FDTD_MULTI_PAIR)
+        return fail(FDTD_ERR_INVALID, "unknown multi-step mode %d", value);
+      s->multi = value;
+      return FDTD_OK;
   }
   return fail(FDTD_ERR_INVALID, "unknown option %d", option);
 }
@@ -759,6 +893,7 @@ int fdtd_get_option(fdtd_sim* s, int option, int* value) {
     case FDTD_OPT_GRAPH_CHUNK: *value = s->graph_chunk; return FDTD_OK;
     case FDTD_OPT_CHECK_EVERY: *value = s->check_every; return FDTD_OK;
     case FDTD_OPT_TIMING: *value = s->timing; return FDTD_OK;
+    case FDTD_OPT_MULTISTEP: *value = s->multi; return FDTD_OK;
   }
   return fail(FDTD_ERR_INVALID, "unknown option %d", option);
 }
@@ -975,7 +1110,7 @@ int fdtd_reset(fdtd_sim* s) {
     CK(cudaMemsetAsync(s->psi_base[set], 0, (size_t)s->psi_elems * s->esz, s->stream));
   CK(cudaMemsetAsync(s->ph, 0, (size_t)s->ph_elems * s->esz, s->stream));
   CK(cudaMemsetAsync(s->phc, 0, (size_t)s->ph_elems * s->esz, s->stream));
-  CK(cudaMemsetAsync(s->tdev, 0, sizeof(int) * 4, s->stream));
+  CK(cudaMemsetAsync(s->tdev, 0, sizeof(int) * 8, s->stream));
   CK(cudaMemsetAsync(s->flags, 0, sizeof(int) * 2, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   s->t = 0;
@@ -1107,6 +1242,7 @@ int fdtd_synchronize(fdtd_sim* s) {
   CK(cudaStreamSynchronize(s->stream));
   CK(cudaGetLastError());
   if ((rc = take_bounds_violation())) return rc;
+  if ((rc = take_wait_error(s))) return rc;
   if (s->check_every > 0) {
     int f[2] = {0, 0};
     CK(cudaMemcpy(f, s->flags, sizeof(f), cudaMemcpyDeviceToHost));
@@ -1171,7 +1307,7 @@ int fdtd_get_phasor(fdtd_sim* s, int plane, void* out) {
   CK(cudaMemcpyAsync(out, (char*)s->ph + s->ph_off[plane] * s->esz, (size_t)(2 * n) * s->esz,
                      cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  return FDTD_OK;
+  return take_wait_error(s);
 }
 
 int fdtd_get_phasors(fdtd_sim* s, void* out) {
@@ -1191,7 +1327,7 @@ int fdtd_get_phasors(fdtd_sim* s, void* out) {
     off += bytes;
   }
   CK(cudaStreamSynchronize(s->stream));
-  return FDTD_OK;
+  return take_wait_error(s);
 }
 
 int fdtd_get_field(fdtd_sim* s, int comp, void* out) {
@@ -1204,7 +1340,7 @@ int fdtd_get_field(fdtd_sim* s, int comp, void* out) {
   CK(cudaMemcpy2DAsync(out, w, s->fld[s->cur][comp], (size_t)s->pitch * s->esz, w,
                        (size_t)s->g.ny * s->g.nz, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  return FDTD_OK;
+  return take_wait_error(s);
 }
 
 int fdtd_set_field(fdtd_sim* s, int comp, const void* in) {
@@ -1712,6 +1848,10 @@ int fdtd_batch_synchronize(fdtd_batch* b) {
   CK(cudaSetDevice(b->device));
   CK(cudaStreamSynchronize(b->stream));
   CK(cudaGetLastError());
+  for (fdtd_sim* s : b->sims) {
+    const int rc = take_wait_error(s);
+    if (rc) return rc;
+  }
   return take_bounds_violation();
 }
 

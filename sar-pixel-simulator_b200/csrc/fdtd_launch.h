@@ -2,6 +2,7 @@
 // the C-ABI implementation.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "fdtd_common.cuh"
@@ -155,6 +156,71 @@ void add_shell_box(ShellBoxes& bl, int x0, int x1, int y0, int y1, int z0, int z
 template <class T>
 void launch_shell_pass(const State<T>& s, const int* tdev, int toff, const ShellBoxes& bl,
                        bool h_pass, cudaStream_t st);
+
+// Pair step (fdtd_pair.cu): two steps per pass, by marches over regions of
+// four kinds. A region is the box x [x0, x1), y [y0, y1), z [z0, z1), cut
+// into gx x gy tiles of sx x sy own cells (the first tile's first computed
+// cell is (xt, yt)) and chunks of zchunk planes; `first` is its first block
+// in the launch.
+struct PairRegion {
+  int x0, x1, xt, sx, gx;
+  int y0, y1, yt, sy, gy;
+  int z0, z1, zchunk;
+  int first;
+};
+struct PairRegions {
+  int n, blocks;
+  float minus0;   // -0, as a value the kernel's compiler does not know
+  PairRegion r[2];
+};
+struct PairPlan {
+  int ok;   // the grid has a plain box worth marching
+  PairRegions plain, zface, yend, xend;
+};
+enum PairKind { kPairPlain = 0, kPairZ, kPairY, kPairX };
+// Tensor maps of the source ex, ey, ez, hx, hy, hz and of ca, cb, for the
+// tiles of each kind.
+struct PairMaps {
+  CUtensorMap m[8];
+};
+struct PairMapSet {
+  PairMaps plain, zface, yend, xend;
+};
+// What the phasors of a pair's first step read, written by the marches
+// instead of the whole fields between the steps: the planes, columns and rows
+// m, m + 1, n - m - 2, n - m - 1 (m = npml) of
+//   z: ex, ey, hx, hy (4, ny, pitch);  y: ex, ez, hx, hz (nz, 4, pitch);
+//   x: ey, ez, hy, hz (nz, ny, 4), of both steps (a row's sector in the
+//      fields holds eight columns).
+template <class T>
+struct PairMid {
+  T* z[4];
+  T* y[4];
+  T* x[2][4];
+};
+// Elements of one component of each.
+template <class T>
+inline void pair_mid_sizes(const State<T>& s, long long (&n)[3]) {
+  n[0] = 4 * s.plane;
+  n[1] = 4LL * s.nz * s.pitch;
+  n[2] = 4LL * s.nz * s.ny;
+}
+
+PairPlan make_pair_plan(int nx, int ny, int nz, int npml, int elem_bytes);
+// Maps of a State's source set; false when the driver cannot make them.
+template <class T>
+bool make_pair_maps(const State<T>& s, PairMapSet* out);
+// The march over the regions of one kind, source set -> destination set;
+// the four may run in any order or side by side. *err (device) is set when
+// a plane's copy did not arrive in time.
+template <class T>
+bool launch_pair(PairKind kind, const State<T>& s, const PairPlan& p, const PairMapSet& maps, const PairMid<T>& mid,
+                 const int* tdev, int toff, int* err, cudaStream_t st);
+// The phasor pass of two steps: of the fields between them (mid: ex, ey,
+// ez, hx, hy, hz) at step toff, then of s's destination set at toff + 1.
+template <class T>
+void launch_phasors_pair(const State<T>& s, const PairMid<T>& mid, const int* tdev, int toff, cudaStream_t st, int g0 = 0,
+                         int ng = 6);
 
 // One transposed step (fdtd_adjoint.cu): s holds E^n in its source E
 // pointers, H^{n+1/2} in its source H pointers and the CPML auxiliaries

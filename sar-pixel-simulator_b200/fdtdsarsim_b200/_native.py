@@ -47,6 +47,10 @@ OPT_SHELL = 11
 SHELL_MARCH = 0
 SHELL_SPLIT = 1
 OPT_BATCH_MODE = 12
+OPT_MULTISTEP = 13
+MULTI_OFF = 0
+MULTI_AUTO = 1
+MULTI_PAIR = 3
 BATCH_SPLIT = 0
 BATCH_STREAMS = 1
 BATCH_QUEUE = 2

@@ -79,7 +79,8 @@ def choose(geom, kernel=None, tile=None, device=0, use_cache=True):
                     'shell': int(hit.get('shell', _SPLIT))}
     k = _native.FDTD_KERNEL_FUSED if kernel is None else int(kernel)
     tx, ty = tile if tile is not None else DEFAULT_TILE
-    return {'kernel': k, 'tile_x': int(tx), 'tile_y': int(ty), 'zchunk': 0, 'slab': 0, 'shell': _SPLIT}
+    return {'kernel': k, 'tile_x': int(tx), 'tile_y': int(ty), 'zchunk': 0, 'slab': 0, 'shell': _SPLIT,
+            'multi': _native.MULTI_AUTO if kernel is None and tile is None else _native.MULTI_OFF}
 
 
 def apply(sim, choice):
@@ -91,6 +92,8 @@ def apply(sim, choice):
         sim.set_option(_native.OPT_ZCHUNK, choice.get('zchunk', 0))
         sim.set_option(_native.OPT_FUSED_SLAB, choice.get('slab', 0))
         sim.set_option(_native.OPT_SHELL, choice.get('shell', _SPLIT))
+        if 'multi' in choice:
+            sim.set_option(_native.OPT_MULTISTEP, choice['multi'])
 
 
 def autotune(geom, device=0, steps=6, candidates=None, save=True):
