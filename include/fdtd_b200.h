@@ -86,7 +86,8 @@ extern "C" {
 
 /* several steps per launch (fdtd_set_option(FDTD_OPT_MULTISTEP, ...)) */
 #define FDTD_MULTI_OFF      0
-#define FDTD_MULTI_AUTO     1 /* by the grid's size: pair or single */
+#define FDTD_MULTI_AUTO     1 /* by the grid's size: resident, pair or single */
+#define FDTD_MULTI_RESIDENT 2 /* every step of fdtd_run in one cooperative launch */
 #define FDTD_MULTI_PAIR     3 /* two steps per pass over the fields; holds a
                                  third field set (single steps where there is
                                  no memory for it, or the grid is too narrow) */

@@ -76,7 +76,7 @@ struct fdtd_sim {
   long long ph_off[24];
   long long ph_elems = 0;
   double* phase = nullptr;
-  int* tdev = nullptr;                   // step counter; [2] stays 0;
+  int* tdev = nullptr;                   // step counter; [2] stays 0; [4], [5] the resident step's barrier;
                                          // [6] set by a kernel when a wait inside it ran out
   int* flags = nullptr;                  // non-finite check: found, step
   int64_t t = 0;
@@ -127,6 +127,7 @@ struct fdtd_sim {
   // this grid or no memory for it), its plan and tensor maps (one set per
   // source set), a third stream for its z-face chunks
   int multi = 0;
+  bool side_by_side = false;             // running among a batch's streams
   int pair_state = 0;
   PairPlan pair;
   PairMapSet pmaps[2];
@@ -441,16 +442,31 @@ int enqueue_pair(fdtd_sim* s, int k, int ph_g0, int ph_ng, cudaEvent_t after_ste
 
 // ph_g0, ph_ng: the phasor plane groups each step accumulates (all six by
 // default; none with ph_ng = 0; the gradient's forward only the upper plane)
-// The path of a run of n steps. FDTD_MULTI_AUTO takes the fastest on the B200
-// (us per step; single, pair):
-//   float  0.97 M cells  49  57      double  0.97 M   84   71
-//          4.32 M       104  91              1.78 M  119   92
-//          14.7 M       230 186              14.7 M  635  328
-// The pair step wins once the plain box outweighs its ends: in float also
-// only on wide grids (91 x 267 x 133 cells: 92 single, 104 pair;
-// 301 x 121 x 121: 116 and 135; 61 x 401 x 201: 125 and 111).
+// The path of a run of n steps. FDTD_MULTI_AUTO takes the fastest of the
+// three on the B200 (us per step; single, resident, pair):
+//   float  0.44 M cells  39  17  40      double  0.44 M   62   27   60
+//          0.97 M        49  28  57              0.97 M   84   59   71
+//          2.71 M        86  76  83              1.78 M  119  101   92
+//          4.32 M       104 117  91              4.32 M  257  226  174
+//          14.7 M       230 376 186              14.7 M  635  769  328
+// The resident step wins while the fields (E, two sets of H, Ca, Cb) stay in
+// the 126 MB L2. The pair step wins once the plain box outweighs its ends:
+// in float also only on wide grids (91 x 267 x 133 cells: 92 single, 104
+// pair; 301 x 121 x 121: 116 and 135; 61 x 401 x 201: 125 and 111).
+constexpr long long kResidentBytes = 128LL << 20;
 constexpr long long kPairCellsFloat = 4000000, kPairCellsDouble = 1500000;
 constexpr int kPairNxFloat = 160;
+
+template <class T>
+bool takes_resident(const fdtd_sim* s, int n) {
+  if (s->kernel != FDTD_KERNEL_FUSED || s->check_every > 0 || n < 2) return false;
+  if (s->multi == FDTD_MULTI_RESIDENT) return true;
+  // members that run side by side: a launch that takes every SM would run
+  // them one after another (10 members of 0.6 to 4 M cells: 507 us per step
+  // against 452)
+  if (s->side_by_side) return false;
+  return s->multi == FDTD_MULTI_AUTO && s->vol * 11 * (long long)sizeof(T) <= kResidentBytes;
+}
 
 bool takes_pair(const fdtd_sim* s) {
   if (s->kernel != FDTD_KERNEL_FUSED || s->check_every > 0) return false;
@@ -462,6 +478,29 @@ bool takes_pair(const fdtd_sim* s) {
 
 template <class T>
 int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
+  if (takes_resident<T>(s, n)) {
+    cudaEvent_t e0 = s->timing ? timing_event(s) : nullptr;
+    cudaEvent_t e1 = s->timing ? timing_event(s) : nullptr;
+    cudaEvent_t e2 = s->timing ? timing_event(s) : nullptr;
+    if (s->timing) s->ev_steps.push_back(n);
+    mark(s, e0);
+    T* const other[3] = {(T*)s->fld[1 - s->cur][3], (T*)s->fld[1 - s->cur][4], (T*)s->fld[1 - s->cur][5]};
+    const bool ok = launch_resident<T>(make_state<T>(s, s->cur, s->cur), other, s->tdev, 0, n, ph_g0, ph_ng,
+                                       (unsigned*)(s->tdev + 4), s->tdev + 6, s->stream);
+    mark(s, e1);
+    mark(s, e2);
+    s->wait_look = true;
+    if (ok) {
+      launch_advance(s->tdev, n, s->stream);
+      CK(cudaGetLastError());
+      return FDTD_OK;
+    }
+    cudaGetLastError();   // a device without cooperative launches: single steps
+    if (s->timing) {
+      s->ev_used -= 3;
+      s->ev_steps.pop_back();
+    }
+  }
   for (int k = 0; k < n; ++k) {
     if (s->timing && s->ev_used + 3 > 3 * 4096) {
       int rc = collect_timing(s);
@@ -1717,7 +1756,9 @@ int batch_run_streams(fdtd_batch* b, int nsteps) {
   CK(cudaEventRecord(b->ev, b->stream));
   for (fdtd_sim* s : b->sims) CK(cudaStreamWaitEvent(s->stream, b->ev, 0));
   for (fdtd_sim* s : b->sims) {
+    s->side_by_side = b->sims.size() > 1;
     const int rc = run_steps<T>(s, nsteps);
+    s->side_by_side = false;
     if (rc) return rc;
   }
   for (size_t m = 0; m < b->sims.size(); ++m) {

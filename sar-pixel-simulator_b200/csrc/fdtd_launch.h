@@ -157,6 +157,29 @@ template <class T>
 void launch_shell_pass(const State<T>& s, const int* tdev, int toff, const ShellBoxes& bl,
                        bool h_pass, cudaStream_t st);
 
+// Resident step (fdtd_resident.cu): many split steps of a small grid in one
+// cooperative launch.
+struct DivMagic {
+  unsigned mul, shift;
+};
+template <class T>
+struct ResidentArgs {
+  State<T> st;       // source == destination: the current set, in place
+  T* other[3];       // hx, hy, hz of the other set
+  long long units;   // warps' units in the grid
+  int gx, gy;        // per row and per column of a plane
+  int ph_units;      // 32-cell units of the largest phasor plane
+  DivMagic per_row, per_plane;   // division by gx and by gy
+  float minus0;      // -0 (fdtd_vecn.cuh: vmul)
+};
+// Enqueues nsteps steps from the step *tdev + toff (their phasors in plane
+// groups ph_g0 .. ph_g0 + ph_ng - 1 included); the run ends on the set it
+// began with. sync: two words of device memory; *err (device) is set when a
+// barrier ran out of time. False: not launched.
+template <class T>
+bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, int toff, int nsteps, int ph_g0,
+                     int ph_ng, unsigned* sync, int* err, cudaStream_t st);
+
 // Pair step (fdtd_pair.cu): two steps per pass, by marches over regions of
 // four kinds. A region is the box x [x0, x1), y [y0, y1), z [z0, z1), cut
 // into gx x gy tiles of sx x sy own cells (the first tile's first computed

@@ -1,5 +1,6 @@
 // fdtd_split.cuh -- the split step's H and E updates of one vector and the
-// phasor update of one cell (fdtd_split.cu).
+// phasor update of one cell, shared by the split passes (fdtd_split.cu) and
+// the resident step (fdtd_resident.cu).
 #pragma once
 
 #include "fdtd_vec.cuh"

@@ -1,5 +1,6 @@
 // fdtd_vecn.cuh -- H and E updates of a vector of V cells with the CPML terms
-// of all faces (the pair step, fdtd_pair.cu).
+// of all faces, shared by the pair step (fdtd_pair.cu) and the resident step
+// (fdtd_resident.cu).
 //
 // The same values as h_vec / e_vec (fdtd_vec.cuh), which the split passes
 // use, with a vector's position (faces, ranges, x-face coefficients) worked

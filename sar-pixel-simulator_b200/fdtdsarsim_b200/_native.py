@@ -50,6 +50,7 @@ OPT_BATCH_MODE = 12
 OPT_MULTISTEP = 13
 MULTI_OFF = 0
 MULTI_AUTO = 1
+MULTI_RESIDENT = 2
 MULTI_PAIR = 3
 BATCH_SPLIT = 0
 BATCH_STREAMS = 1

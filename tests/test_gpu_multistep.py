@@ -29,6 +29,17 @@ PAIR = [
 ]
 
 
+# grids down to the smallest, rows of every unit width, odd and even runs
+RESIDENT = [
+    (27, 25, 23, 10, 12, 7, 'float32'),
+    (7, 8, 9, 2, 4, 6, 'float32'),
+    (150, 33, 26, 10, 20, 4, 'float32'),
+    (64, 70, 31, 7, 14, 5, 'float32'),
+    (33, 23, 25, 10, 12, 6, 'float64'),
+    (45, 41, 29, 10, 24, 5, 'float64'),
+]
+
+
 def _multi(pc, ca, cb, inc, mode, phasor_mode=0):
     sim = native_for(pc, _native.FDTD_KERNEL_FUSED, (32, 4), phasor_mode, shell=_native.SHELL_SPLIT)
     sim.set_option(_native.OPT_MULTISTEP, mode)
@@ -44,8 +55,10 @@ def _assert_matches(orc, sim):
         assert bits_equal(sim.get_phasor(k), orc.ph[name]), name
 
 
-@pytest.mark.parametrize('case,mode', [(c, _native.MULTI_PAIR) for c in PAIR],
-                         ids=lambda c: 'x'.join(map(str, c)) if isinstance(c, tuple) else 'pair')
+@pytest.mark.parametrize('case,mode', [(c, _native.MULTI_PAIR) for c in PAIR]
+                         + [(c, _native.MULTI_RESIDENT) for c in RESIDENT],
+                         ids=lambda c: 'x'.join(map(str, c)) if isinstance(c, tuple) else
+                         {_native.MULTI_PAIR: 'pair', _native.MULTI_RESIDENT: 'resident'}[c])
 def test_multi_step_matches_oracle(case, mode):
     """A run, then a second one from the field set that the first left;
     between them odd and even counts, injection ending inside the first."""
