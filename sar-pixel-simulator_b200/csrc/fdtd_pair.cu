@@ -29,9 +29,12 @@
 //           uniform over a plane (32 x 12)
 //   y ends  the rows at either y end, same x range: y and z faces (16 x 14)
 //   x ends  the columns at either x end, all y, all z: every face. Tiles of
-//           32 cells (128 bytes) by 32 (float) or 16 (double) rows: rows of
-//           an x face are short, and a wide tile would march mostly plain
-//           cells with the general update.
+//           128-byte rows by 32 rows: the rows of an x face are short, and a
+//           wide tile would march mostly plain cells with the general update.
+//           (Tiles turned so that a warp is one column of vectors, where an x
+//           face is uniform over a warp, ran fewer instructions, but the face
+//           warps kept the others waiting at the barriers: 183 us against
+//           148 at 101 x 381 x 381.)
 // The z-face, x-face and y-face CPML auxiliaries of the two steps stay in
 // registers between them (read from the source set, written to the
 // destination set once).
@@ -46,10 +49,10 @@
 // L2.
 //
 // Measured (float, us per step, single steps and pairs, phasors included):
-// 203 x 761 x 761 cells 1485 and 924; 101 x 381 x 381 243 and 185; double,
-// 101 x 381 x 381 650 and 347. At 203 x 761 x 761 the plain march takes 980 us
-// per pair (6.0 TB/s; 5.9 GB, of which 10 % is halo), the z faces 310, the
-// x ends 490, the y ends 130; those three are bound by instructions and
+// 203 x 761 x 761 cells 1485 and 923; 101 x 381 x 381 243 and 184; double,
+// 101 x 381 x 381 650 and 322. At 203 x 761 x 761 the plain march takes 973 us
+// per pair (6.0 TB/s; 5.9 GB, of which 10 % is halo), the z faces 302, the
+// x ends 463, the y ends 123; those three are bound by instructions and
 // latency (IPC 1.3 to 1.5 at one block of 12 to 16 warps per SM), not by HBM.
 #include <algorithm>
 #include <cstring>
@@ -65,36 +68,28 @@ namespace {
 
 constexpr unsigned long long kWaitNs = 2000000000ull;   // one mbarrier wait gives up after this long
 
-// A tile of TR warps, elements T, V cells per thread, with the CPML faces it
-// can meet (none: a plain tile). A row is L threads of one warp, the tile 32
-// TR / L rows; or, turned (kT), a warp is one column of vectors, its lanes 32
-// rows: what depends on x is then uniform over a warp. Shared memory: E ring
+// A tile of L threads per row and TR warps, elements T, V cells per thread,
+// with the CPML faces it can meet (none: a plain tile). Shared memory: E ring
 // (3 planes of 3 components of kRows + 1 rows), ring of H, Ca, Cb (2 planes
-// of 5 components of kRows rows), the exchange area (H1, E1 twice, H2), the
-// five mbarriers. A turned tile's rows are 128 bytes, swizzled (16-byte
-// pieces of eight consecutive rows spread over the banks).
-template <class T_, int V_, int L_, int TR_, bool kX_, bool kY_, bool kZ_, bool kT_ = false>
+// of 5 components of kRows rows), exchange rows x and z of H1, E1 (two
+// buffers), H2; the five mbarriers.
+template <class T_, int V_, int L_, int TR_, bool kX_, bool kY_, bool kZ_>
 struct PairTile {
   using T = T_;
   static constexpr int V = V_, L = L_, TR = TR_;
-  static constexpr bool kX = kX_, kY = kY_, kZ = kZ_, kT = kT_, kEdge = kX || kY || kZ;
-  static constexpr int kCells = kT ? TR * V : L * V;   // cells of a row
-  static constexpr int kRows = kT ? 32 : 32 * TR / L;
+  static constexpr bool kX = kX_, kY = kY_, kZ = kZ_, kEdge = kX || kY || kZ;
+  static constexpr int kCells = L * V;   // cells of a row
+  static constexpr int kRows = 32 * TR / L;
   static constexpr int kRowBytes = kCells * (int)sizeof(T);
-  static constexpr int kEComp = kT ? (kRows + 8) * kRowBytes : (kRows + 1) * kRowBytes;   // (1024-byte steps)
-  static constexpr int kHComp = kRows * kRowBytes;
-  static constexpr int kEBytes = 3 * (kRows + 1) * kRowBytes, kHBytes = 5 * kHComp;   // what arrives per plane
-  static constexpr int kHRing = 9 * kEComp, kXchAt = kHRing + 10 * kHComp;
-  // one exchange buffer: two vectors per thread, or (turned) two cells
-  static constexpr int kXch = kT ? 2 * 32 * TR * (int)sizeof(T) : 2 * kRows * kRowBytes;
-  // a turned tile's results leave through shared memory, in whole rows
-  static constexpr int kOutAt = kXchAt + 4 * kXch;
-  static constexpr int kBars = kOutAt + (kT ? 6 * kHComp : 0);
+  static constexpr int kEComp = (kRows + 1) * kRowBytes, kHComp = kRows * kRowBytes;
+  static constexpr int kEBytes = 3 * kEComp, kHBytes = 5 * kHComp;   // a plane of each ring
+  static constexpr int kHRing = 3 * kEBytes, kXchAt = kHRing + 2 * kHBytes;
+  static constexpr int kXch = 2 * kHComp;
+  static constexpr int kBars = kXchAt + 4 * kXch;
   static constexpr int kBytes = kBars + 64;
   // recomputed cells at either x end: two, rounded up to the 16 bytes a copy starts on
   static constexpr int kHalo = 16 / (int)sizeof(T);
   static constexpr int kOutX = kCells - 2 * kHalo, kOutY = kRows - 3;
-  static_assert(!kT || kRowBytes == 128, "a turned tile's row is one swizzle span");
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -148,9 +143,9 @@ struct PairCarry {
 // The kinds of tile a warp computes as on a plane where it meets no boundary,
 // or only an x face.
 template <class C>
-using PairPlain = PairTile<typename C::T, C::V, C::L, C::TR, false, false, false, C::kT>;
+using PairPlain = PairTile<typename C::T, C::V, C::L, C::TR, false, false, false>;
 template <class C>
-using PairOnlyX = PairTile<typename C::T, C::V, C::L, C::TR, C::kX, false, false, C::kT>;
+using PairOnlyX = PairTile<typename C::T, C::V, C::L, C::TR, C::kX, false, false>;
 
 template <class C>
 __global__ void __launch_bounds__(32 * C::TR, 1)
@@ -163,8 +158,7 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
   extern __shared__ __align__(1024) unsigned char smem[];
   const unsigned base = smem_u32(smem);
   const unsigned bars = base + C::kBars;   // E slots 0..2, then HC slots 0..1
-  const int lane = C::kT ? threadIdx.x >> 5 : threadIdx.x % C::L;   // vector of the row
-  const int r = C::kT ? threadIdx.x & 31 : threadIdx.x / C::L;
+  const int lane = threadIdx.x % C::L, r = threadIdx.x / C::L;
 
   int bid = blockIdx.x;
   const PairRegion& b = rg.r[rg.n > 1 && bid >= rg.r[1].first ? 1 : 0];
@@ -206,14 +200,14 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
 
   auto issue_e = [&](int z) {
     const int slot = (z - zs) % 3;
-    const unsigned bar = bars + 8 * slot, dst = base + slot * 3 * C::kEComp;
+    const unsigned bar = bars + 8 * slot, dst = base + slot * C::kEBytes;
     mbar_expect(bar, C::kEBytes);
 #pragma unroll
     for (int k = 0; k < 3; ++k) tma_plane(dst + k * C::kEComp, &maps.m[k], bar, xt, yt, z);
   };
   auto issue_hc = [&](int z) {
     const int slot = (z - zs) & 1;
-    const unsigned bar = bars + 24 + 8 * slot, dst = base + C::kHRing + slot * 5 * C::kHComp;
+    const unsigned bar = bars + 24 + 8 * slot, dst = base + C::kHRing + slot * C::kHBytes;
     mbar_expect(bar, C::kHBytes);
 #pragma unroll
     for (int k = 0; k < 5; ++k) tma_plane(dst + k * C::kHComp, &maps.m[3 + k], bar, xt, yt, z);
@@ -226,75 +220,23 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     if (zs + 2 <= ze) issue_e(zs + 2);
   }
 
-  // where a cell of a row lies in a ring component
-  auto place = [&](int row, int cell) {
-    const int o = cell * kSz;
-    return row * C::kRowBytes + (C::kT ? (((o >> 4) ^ (row & 7)) << 4) + (o & 15) : o);
-  };
-  const int at = place(r, lane * V), up_at = place(r + 1, lane * V);
-  const int right = place(r, C::kT && lane + 1 < C::TR ? (lane + 1) * V : lane * V);   // turned: the next vector
-  // an exchange buffer holds, per thread, the vectors x and z of a field
-  // (for the rows above and below), or, turned, the cells y and z that the
-  // next warp needs (rows then meet by shuffle). Rows and vectors at the
-  // tile's edge read a stand-in: they compute nothing that counts.
-  constexpr int kHalf = C::kXch / 2 / kSz;
-  const int own_at = C::kT ? (int)threadIdx.x : at / kSz;
-  const int dn = C::kT ? (lane > 0 ? own_at - 32 : own_at) : ((r > 0 ? r - 1 : 0) * C::kCells + lane * V);
-  const int up = C::kT ? (lane + 1 < C::TR ? own_at + 32 : own_at) : ((r < NR - 1 ? r + 1 : r) * C::kCells + lane * V);
+  // this thread's place in a tile plane, and those of the rows below and
+  // above (rows at the tile's edge read a stand-in: they compute nothing
+  // that counts), in elements
+  const int at = r * C::kCells + lane * V;
+  const int dn = r > 0 ? at - C::kCells : at, up = r < NR - 1 ? at + C::kCells : at;
+  constexpr int kHalf = C::kHComp / kSz;   // the second row set of an exchange buffer
   auto xch = [&](int k) { return reinterpret_cast<T*>(smem + C::kXchAt + k * C::kXch); };
-  // H of the row below (x, z) and of the vector to the left (y, z)
-  auto h_out = [&](T* w, const T (&hx)[V], const T (&hy)[V], const T (&hz)[V]) {
-    if constexpr (C::kT) {
-      w[own_at] = hy[V - 1];
-      w[kHalf + own_at] = hz[V - 1];
-    } else {
-      sts(w + own_at, hx);
-      sts(w + kHalf + own_at, hz);
-    }
+  // H of the row below (x, z) and the previous lane's last cell (y, z)
+  auto h_in = [&](const T* w, const T (&hy)[V], const T (&hz)[V], T (&hxy)[V], T (&hzy)[V], T& hyp, T& hzp) {
+    lds(hxy, w + dn);
+    lds(hzy, w + kHalf + dn);
+    hyp = __shfl_up_sync(kAll, hy[V - 1], 1, C::L);
+    hzp = __shfl_up_sync(kAll, hz[V - 1], 1, C::L);
   };
-  auto h_in = [&](const T* w, const T (&hx)[V], const T (&hy)[V], const T (&hz)[V], T (&hxy)[V], T (&hzy)[V], T& hyp,
-                  T& hzp) {
-    if constexpr (C::kT) {
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        hxy[j] = __shfl_up_sync(kAll, hx[j], 1);
-        hzy[j] = __shfl_up_sync(kAll, hz[j], 1);
-      }
-      hyp = w[dn];
-      hzp = w[kHalf + dn];
-    } else {
-      lds(hxy, w + dn);
-      lds(hzy, w + kHalf + dn);
-      hyp = __shfl_up_sync(kAll, hy[V - 1], 1, C::L);
-      hzp = __shfl_up_sync(kAll, hz[V - 1], 1, C::L);
-    }
-  };
-  // E of the row above (x, z) and of the vector to the right (y, z)
-  auto e_out = [&](T* w, const T (&ex)[V], const T (&ey)[V], const T (&ez)[V]) {
-    if constexpr (C::kT) {
-      w[own_at] = ey[0];
-      w[kHalf + own_at] = ez[0];
-    } else {
-      sts(w + own_at, ex);
-      sts(w + kHalf + own_at, ez);
-    }
-  };
-  auto e_in = [&](const T* w, const T (&ex)[V], const T (&ey)[V], const T (&ez)[V], T (&exy)[V], T (&ezy)[V], T& eyn,
-                  T& ezn) {
-    if constexpr (C::kT) {
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        exy[j] = __shfl_down_sync(kAll, ex[j], 1);
-        ezy[j] = __shfl_down_sync(kAll, ez[j], 1);
-      }
-      eyn = w[up];
-      ezn = w[kHalf + up];
-    } else {
-      lds(exy, w + up);
-      lds(ezy, w + kHalf + up);
-      eyn = __shfl_down_sync(kAll, ey[0], 1, C::L);
-      ezn = __shfl_down_sync(kAll, ez[0], 1, C::L);
-    }
+  auto out = [&](T* w, const T (&a)[V], const T (&b)[V]) {
+    sts(w + at, a);
+    sts(w + kHalf + at, b);
   };
 
   // the vector's cells in the phasors' x columns
@@ -306,24 +248,6 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
       if (k < 0) continue;
       const unsigned i = (unsigned)((z * s.ny + p.y) * 4 + k);
       stc(to[0] + i, a0[j]); stc(to[1] + i, a1[j]); stc(to[2] + i, a2[j]); stc(to[3] + i, a3[j]);
-    }
-  };
-
-  // the results of plane zo from the turned tile's staging area, a row of
-  // threads per row of cells
-  auto flush = [&](int zo) {
-    const int fr = threadIdx.x / (C::kCells / V), fl = threadIdx.x % (C::kCells / V);
-    const int x = xt + fl * V, y = yt + fr;
-    if (x >= xo && x < min(b.x1, xo + b.sx) && y >= yo && y < min(b.y1, yo + b.sy)) {
-      const unsigned char* const q = smem + C::kOutAt + place(fr, fl * V);
-      const unsigned i = (unsigned)zo * P + (unsigned)(y * s.pitch + x);
-      T* const to[6] = {s.ohx, s.ohy, s.ohz, s.oex, s.oey, s.oez};
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        T v[V];
-        lds(v, reinterpret_cast<const T*>(q + k * C::kHComp));
-        stg(to[k] + i, v);
-      }
     }
   };
 
@@ -359,34 +283,29 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
         ep ^= 1u << en;
       }
       good = good && mbar_wait(bars + 24 + 8 * (k & 1), (k >> 1) & 1);
-      const unsigned char* const E0 = smem + es * 3 * C::kEComp;
-      const unsigned char* const E1 = smem + en * 3 * C::kEComp + at;
-      const unsigned char* const HC = smem + C::kHRing + (k & 1) * 5 * C::kHComp + at;
-      auto cell = [](const unsigned char* q) { return reinterpret_cast<const T*>(q); };
-      T exz[V], eyz[V], exy[V], ezy[V], eyn, ezn;
-      lds(d.ex, cell(E0 + at));
-      lds(d.ey, cell(E0 + C::kEComp + at));
-      lds(d.ez, cell(E0 + 2 * C::kEComp + at));
-      lds(exy, cell(E0 + up_at));
-      lds(ezy, cell(E0 + 2 * C::kEComp + up_at));
-      lds(exz, cell(E1));
-      lds(eyz, cell(E1 + C::kEComp));
-      lds(d.hx, cell(HC));
-      lds(d.hy, cell(HC + C::kHComp));
-      lds(d.hz, cell(HC + 2 * C::kHComp));
-      lds(d.ca, cell(HC + 3 * C::kHComp));
-      lds(d.cb, cell(HC + 4 * C::kHComp));
-      if constexpr (C::kT) {
-        eyn = *cell(E0 + C::kEComp + right);
-        ezn = *cell(E0 + 2 * C::kEComp + right);
-      } else {
-        eyn = __shfl_down_sync(kAll, d.ey[0], 1, C::L);
-        ezn = __shfl_down_sync(kAll, d.ez[0], 1, C::L);
-      }
+      const T* const E0 = reinterpret_cast<const T*>(smem + es * C::kEBytes) + at;
+      const T* const E1 = reinterpret_cast<const T*>(smem + en * C::kEBytes) + at;
+      const T* const HC = reinterpret_cast<const T*>(smem + C::kHRing + (k & 1) * C::kHBytes) + at;
+      constexpr int kEc = C::kEComp / kSz, kHc = C::kHComp / kSz;
+      T exz[V], eyz[V], exy[V], ezy[V];
+      lds(d.ex, E0);
+      lds(d.ey, E0 + kEc);
+      lds(d.ez, E0 + 2 * kEc);
+      lds(exy, E0 + C::kCells);
+      lds(ezy, E0 + 2 * kEc + C::kCells);
+      lds(exz, E1);
+      lds(eyz, E1 + kEc);
+      lds(d.hx, HC);
+      lds(d.hy, HC + kHc);
+      lds(d.hz, HC + 2 * kHc);
+      lds(d.ca, HC + 3 * kHc);
+      lds(d.cb, HC + 4 * kHc);
+      const T eyn = __shfl_down_sync(kAll, d.ey[0], 1, C::L);
+      const T ezn = __shfl_down_sync(kAll, d.ez[0], 1, C::L);
       if (easy1) pair_h<PairPlain<C>>(s, p, z, t, d.ex, d.ey, d.ez, exz, eyz, exy, ezy, eyn, ezn, d.hx, d.hy, d.hz, d.ph);
       else if (xonly1) pair_h<PairOnlyX<C>>(s, p, z, t, d.ex, d.ey, d.ez, exz, eyz, exy, ezy, eyn, ezn, d.hx, d.hy, d.hz, d.ph);
       else pair_h<C>(s, p, z, t, d.ex, d.ey, d.ez, exz, eyz, exy, ezy, eyn, ezn, d.hx, d.hy, d.hz, d.ph);
-      h_out(xch(0), d.hx, d.hy, d.hz);
+      out(xch(0), d.hx, d.hz);
     }
     __syncthreads();
     // every thread has read plane z of the rings: their slots take new planes
@@ -394,16 +313,15 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
       if (z + 3 <= ze) issue_e(z + 3);
       if (z + 2 <= zl) issue_hc(z + 2);
     }
-    if (C::kT && z - 2 >= z0) flush(z - 2);
     if (first) {
       T hxy[V], hzy[V], hyp, hzp;
-      h_in(xch(0), d.hx, d.hy, d.hz, hxy, hzy, hyp, hzp);
+      h_in(xch(0), d.hy, d.hz, hxy, hzy, hyp, hzp);
       if (easy1)
         pair_e<PairPlain<C>>(s, p, z, t, d.hx, d.hy, d.hz, g.hx, g.hy, hxy, hzy, hyp, hzp, d.ca, d.cb, d.ex, d.ey, d.ez,
                              d.pe);
       else if (xonly1) pair_e<PairOnlyX<C>>(s, p, z, t, d.hx, d.hy, d.hz, g.hx, g.hy, hxy, hzy, hyp, hzp, d.ca, d.cb, d.ex, d.ey, d.ez, d.pe);
       else pair_e<C>(s, p, z, t, d.hx, d.hy, d.hz, g.hx, g.hy, hxy, hzy, hyp, hzp, d.ca, d.cb, d.ex, d.ey, d.ez, d.pe);
-      e_out(xch(1 + (k & 1)), d.ex, d.ey, d.ez);
+      out(xch(1 + (k & 1)), d.ex, d.ez);
       if (own && z >= z0 && z < z1) {
         const int mz = mid_slot(z, nz);
         if (mz >= 0) {
@@ -421,8 +339,12 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     const bool second = k >= 1;
     T h2z[V];
     if (second) {
-      T exy[V], ezy[V], eyn, ezn;
-      e_in(xch(1 + ((k - 1) & 1)), g.ex, g.ey, g.ez, exy, ezy, eyn, ezn);
+      T exy[V], ezy[V];
+      const T* const w = xch(1 + ((k - 1) & 1));
+      lds(exy, w + up);
+      lds(ezy, w + kHalf + up);
+      const T eyn = __shfl_down_sync(kAll, g.ey[0], 1, C::L);
+      const T ezn = __shfl_down_sync(kAll, g.ez[0], 1, C::L);
 #pragma unroll
       for (int j = 0; j < V; ++j) { d.h2x[j] = g.hx[j]; d.h2y[j] = g.hy[j]; h2z[j] = g.hz[j]; }
       if (easy2)
@@ -430,12 +352,12 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
                              g.ph);
       else if (xonly2) pair_h<PairOnlyX<C>>(s, p, z - 1, t + 1, g.ex, g.ey, g.ez, d.ex, d.ey, exy, ezy, eyn, ezn, d.h2x, d.h2y, h2z, g.ph);
       else pair_h<C>(s, p, z - 1, t + 1, g.ex, g.ey, g.ez, d.ex, d.ey, exy, ezy, eyn, ezn, d.h2x, d.h2y, h2z, g.ph);
-      h_out(xch(3), d.h2x, d.h2y, h2z);
+      out(xch(3), d.h2x, h2z);
     }
     __syncthreads();
     if (second) {
       T hxy[V], hzy[V], hyp, hzp;
-      h_in(xch(3), d.h2x, d.h2y, h2z, hxy, hzy, hyp, hzp);
+      h_in(xch(3), d.h2y, h2z, hxy, hzy, hyp, hzp);
       if (easy2)
         pair_e<PairPlain<C>>(s, p, z - 1, t + 1, d.h2x, d.h2y, h2z, g.h2x, g.h2y, hxy, hzy, hyp, hzp, g.ca, g.cb, g.ex,
                              g.ey, g.ez, g.pe);
@@ -443,17 +365,10 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
                      g.ez, g.pe);
       else pair_e<C>(s, p, z - 1, t + 1, d.h2x, d.h2y, h2z, g.h2x, g.h2y, hxy, hzy, hyp, hzp, g.ca, g.cb, g.ex, g.ey,
                      g.ez, g.pe);
-      if constexpr (C::kT) {
-        auto out = [&](int k, const T (&v)[V]) { sts(reinterpret_cast<T*>(smem + C::kOutAt + k * C::kHComp + at), v); };
-        out(0, d.h2x); out(1, d.h2y); out(2, h2z);
-        out(3, g.ex); out(4, g.ey); out(5, g.ez);
-      }
       if (own && z - 1 >= z0) {
-        if constexpr (!C::kT) {
-          const unsigned i = (unsigned)(z - 1) * P + p.kx;
-          stg(s.ohx + i, d.h2x); stg(s.ohy + i, d.h2y); stg(s.ohz + i, h2z);
-          stg(s.oex + i, g.ex); stg(s.oey + i, g.ey); stg(s.oez + i, g.ez);
-        }
+        const unsigned i = (unsigned)(z - 1) * P + p.kx;
+        stg(s.ohx + i, d.h2x); stg(s.ohy + i, d.h2y); stg(s.ohz + i, h2z);
+        stg(s.oex + i, g.ex); stg(s.oey + i, g.ey); stg(s.oez + i, g.ez);
         if (C::kX && mid_x) x_columns(z - 1, mid.x[1], g.ey, g.ez, d.h2y, h2z);
         if (C::kEdge && !easy2) {
           auto store = [](T (&v)[V], const T*, T* to) { stg(to, v); };
@@ -469,10 +384,6 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     plane(z, A, B);
     if (z < z1) plane(z + 1, B, A);
   }
-  if (C::kT) {
-    __syncthreads();
-    flush(z1 - 1);
-  }
   if (!good) *err = 1;   // a copy did not arrive within the time limit
 }
 
@@ -481,7 +392,7 @@ template <class T> constexpr int kWide = 16 / (int)sizeof(T);
 template <class T> using PlainTile = PairTile<T, kWide<T>, 32, 16, false, false, false>;
 template <class T> using ZTile = PairTile<T, kWide<T>, 32, 12, false, false, true>;
 template <class T> using YTile = PairTile<T, kWide<T> / 2, 32, 14, false, true, true>;
-template <class T> using XTile = PairTile<T, kWide<T> / 2, 32, 16, true, true, true, true>;
+template <class T> using XTile = PairTile<T, kWide<T> / 2, 16, 16, true, true, true>;
 constexpr int kPairSlots = 148;   // blocks in flight
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -502,7 +413,7 @@ EncodeFn encode_fn() {
 // A map of one (nz, ny, pitch) array for tiles of `cells` x box_rows of one
 // plane; parts outside the array read as zeros.
 template <class T>
-bool encode(CUtensorMap* map, const void* p, const State<T>& s, int cells, int box_rows, bool swizzle) {
+bool encode(CUtensorMap* map, const void* p, const State<T>& s, int cells, int box_rows) {
   static const EncodeFn fn = encode_fn();
   if (!fn) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)s.pitch, (cuuint64_t)s.ny, (cuuint64_t)s.nz};
@@ -510,8 +421,7 @@ bool encode(CUtensorMap* map, const void* p, const State<T>& s, int cells, int b
   const cuuint32_t box[3] = {(cuuint32_t)cells, (cuuint32_t)box_rows, 1};
   const cuuint32_t one[3] = {1, 1, 1};
   return fn(map, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
-            const_cast<void*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+            const_cast<void*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -519,7 +429,7 @@ template <class C>
 bool tile_maps(const State<typename C::T>& s, PairMaps* out) {
   const void* f[8] = {s.iex, s.iey, s.iez, s.ihx, s.ihy, s.ihz, s.ca, s.cb};
   for (int k = 0; k < 8; ++k)
-    if (!encode(&out->m[k], f[k], s, C::kCells, C::kRows + (k < 3 ? 1 : 0), C::kT)) return false;
+    if (!encode(&out->m[k], f[k], s, C::kCells, C::kRows + (k < 3 ? 1 : 0))) return false;
   return true;
 }
 
