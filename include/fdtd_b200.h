@@ -285,6 +285,15 @@ int fdtd_grad_forward(fdtd_sim *s, int checkpoint_every);
 int fdtd_grad_backward(fdtd_sim *s, const double *dj_dre, const double *dj_dim, int nz_out,
                        double *grad_ca, double *grad_cb);
 
+/* The same with the gradients taken on to the relative permittivity and
+ * conductivity of the first nz_out planes, whose values (nz_out, ny, nx
+ * float64) the caller gives: dJ/deps_r and dJ/dsigma, (nz_out, ny, nx)
+ * float64, through Ca and Cb as compute_material_arrays
+ * (materials/materials.py:23-68) makes them. */
+int fdtd_grad_backward_eps_sigma(fdtd_sim *s, const double *dj_dre, const double *dj_dim, int nz_out,
+                                 const double *eps_r, const double *sigma, double *grad_eps_r,
+                                 double *grad_sigma);
+
 /* ---- batched sweep --------------------------------------------------------
  * Several simulations (uneven grids, one device, one element type) advanced
  * together: every time step runs the H pass, the E pass and the phasor pass

@@ -861,4 +861,45 @@ template void launch_adjoint_step<float>(const State<float>&, const Adj<float>&,
 template void launch_adjoint_step<double>(const State<double>&, const Adj<double>&, int, bool,
                                           cudaStream_t);
 
+// dJ/deps_r and dJ/dsigma of the material block's cells from dJ/dCa, dJ/dCb
+// (pitched): the closed form of compute_material_arrays (Ca = (1 - x) / (1 + x),
+// Cb = (dt / (eps_r eps0 dx)) / (1 + x), x = sigma dt / (2 eps_r eps0);
+// materials/materials.py:45-63), operation for operation as
+// adjoint.ca_cb_partials evaluates it in float64. eps, sig, ge, gs: (rows,
+// nx) packed. HBM-bound, one pass over 48 bytes a cell. On the host the
+// combination took 20 ms of a 109 ms gradient (584 thousand cells).
+__global__ void __launch_bounds__(256) k_grad_eps_sigma(int nx, long long rows, int pitch, double dt, double dx,
+                                                        const double* __restrict__ gca,
+                                                        const double* __restrict__ gcb,
+                                                        const double* __restrict__ eps,
+                                                        const double* __restrict__ sig, double* __restrict__ ge,
+                                                        double* __restrict__ gs) {
+  using M = R<double>;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= nx) return;
+  for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
+    const long long k = r * nx + x, i = r * pitch + x;
+    const double e = eps[k], a = gca[i], b = gcb[i];
+    const double perm = M::mul(e, 8.8541878128e-12);
+    const double den = M::mul(2.0, perm);
+    const double xl = M::div(M::mul(sig[k], dt), den);
+    const double x_de = M::div(-xl, e), x_ds = M::div(dt, den);
+    const double p = M::add(1.0, xl), p2 = M::mul(p, p);
+    const double ca_x = M::div(-2.0, p2);
+    const double cb0 = M::div(dt, M::mul(perm, dx));
+    const double ca_e = M::mul(ca_x, x_de), ca_s = M::mul(ca_x, x_ds);
+    const double cb_e = M::sub(M::div(M::div(-cb0, e), p), M::mul(M::div(cb0, p2), x_de));
+    const double cb_s = M::mul(M::div(-cb0, p2), x_ds);
+    ge[k] = M::add(M::mul(a, ca_e), M::mul(b, cb_e));
+    gs[k] = M::add(M::mul(a, ca_s), M::mul(b, cb_s));
+  }
+}
+
+void launch_grad_eps_sigma(int nx, long long rows, int pitch, double dt, double dx, const double* gca,
+                           const double* gcb, const double* eps, const double* sig, double* ge, double* gs,
+                           cudaStream_t st) {
+  const dim3 grd((nx + 255) / 256, (unsigned)(rows < 65535 ? rows : 65535), 1);
+  k_grad_eps_sigma<<<grd, 256, 0, st>>>(nx, rows, pitch, dt, dx, gca, gcb, eps, sig, ge, gs);
+}
+
 }  // namespace fdtd

@@ -1986,7 +1986,7 @@ Psi<T> psi_view(const fdtd_sim* s, T* base) {
 }
 
 template <class T>
-int grad_backward(fdtd_sim* s, int nz_out, double* out_ca, double* out_cb) {
+int grad_backward(fdtd_sim* s, int nz_out, double* out_ca, double* out_cb, const double* eps, const double* sigma) {
   const int nt = s->g.nt, every = s->grad_every;
   const long long vol = s->vol, se = state_elems(s);
   T* seg = static_cast<T*>(s->grad_seg);
@@ -2073,6 +2073,23 @@ int grad_backward(fdtd_sim* s, int nz_out, double* out_ca, double* out_cb) {
   if (e != cudaSuccess) return fail(FDTD_ERR_CUDA, "adjoint sweep: %s", cudaGetErrorString(e));
   int rc = set_step(s, nt);   // the fields still hold the forward solve's last state
   if (rc) return rc;
+  if (eps) {   // with respect to eps_r and sigma, made on the device
+    const long long rows = (long long)nz_out * s->g.ny;
+    const size_t n = (size_t)rows * s->g.nx;
+    // in the segment's slots, which the sweep is done with: 32 bytes a cell
+    // of their 2 * every * (6 fields and the psi) >= 48
+    double* d = static_cast<double*>(s->grad_seg);
+    CK(cudaMemcpyAsync(d, eps, n * sizeof(double), cudaMemcpyHostToDevice, s->stream));
+    CK(cudaMemcpyAsync(d + n, sigma, n * sizeof(double), cudaMemcpyHostToDevice, s->stream));
+    if (n)
+      launch_grad_eps_sigma(s->g.nx, rows, s->pitch, s->g.timestep, s->g.cell_size, s->grad_ca, s->grad_cb, d, d + n,
+                            d + 2 * n, d + 3 * n, s->stream);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(out_ca, d + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(out_cb, d + 3 * n, n * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    return FDTD_OK;
+  }
   // the first nz_out planes of the gradients, without the row padding
   const size_t row = (size_t)s->g.nx * sizeof(double);
   const size_t spitch = (size_t)s->pitch * sizeof(double);
@@ -2124,8 +2141,8 @@ int fdtd_grad_forward(fdtd_sim* s, int checkpoint_every) {
   return FDTD_OK;
 }
 
-int fdtd_grad_backward(fdtd_sim* s, const double* dj_dre, const double* dj_dim, int nz_out,
-                       double* grad_ca, double* grad_cb) {
+static int grad_backward_call(fdtd_sim* s, const double* dj_dre, const double* dj_dim, int nz_out, const double* eps,
+                              const double* sigma, double* grad_ca, double* grad_cb) {
   DeviceGuard device_guard;   // the caller's current device is restored on return
   int rc = check_sim(s);
   if (rc) return rc;
@@ -2158,10 +2175,21 @@ int fdtd_grad_backward(fdtd_sim* s, const double* dj_dre, const double* dj_dim, 
   CK(cudaMemsetAsync(s->grad_cb, 0, gb, s->stream));
   CK(cudaMemcpyAsync(s->grad_gre, dj_dre, pb, cudaMemcpyHostToDevice, s->stream));
   CK(cudaMemcpyAsync(s->grad_gim, dj_dim, pb, cudaMemcpyHostToDevice, s->stream));
-  rc = s->g.dtype == FDTD_F32 ? grad_backward<float>(s, nz_out, grad_ca, grad_cb)
-                              : grad_backward<double>(s, nz_out, grad_ca, grad_cb);
+  rc = s->g.dtype == FDTD_F32 ? grad_backward<float>(s, nz_out, grad_ca, grad_cb, eps, sigma)
+                              : grad_backward<double>(s, nz_out, grad_ca, grad_cb, eps, sigma);
   s->grad_forward_done = false;
   return rc;
+}
+
+int fdtd_grad_backward(fdtd_sim* s, const double* dj_dre, const double* dj_dim, int nz_out,
+                       double* grad_ca, double* grad_cb) {
+  return grad_backward_call(s, dj_dre, dj_dim, nz_out, nullptr, nullptr, grad_ca, grad_cb);
+}
+
+int fdtd_grad_backward_eps_sigma(fdtd_sim* s, const double* dj_dre, const double* dj_dim, int nz_out,
+                                 const double* eps_r, const double* sigma, double* grad_eps_r, double* grad_sigma) {
+  if (s && (!eps_r || !sigma || !grad_eps_r || !grad_sigma)) return fail(FDTD_ERR_INVALID, "null eps/sigma or gradient");
+  return grad_backward_call(s, dj_dre, dj_dim, nz_out, eps_r, sigma, grad_eps_r, grad_sigma);
 }
 
 }  // extern "C"

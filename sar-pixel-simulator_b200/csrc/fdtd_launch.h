@@ -255,6 +255,12 @@ void launch_adjoint_first(const State<T>& s, const Adj<T>& a, int t, cudaStream_
 template <class T>
 void launch_adjoint_step(const State<T>& s, const Adj<T>& a, int t, bool first, cudaStream_t st);
 
+// dJ/deps_r, dJ/dsigma (packed rows of nx) from dJ/dCa, dJ/dCb (pitched) and
+// the block's eps_r, sigma (packed); all float64, device.
+void launch_grad_eps_sigma(int nx, long long rows, int pitch, double dt, double dx, const double* gca,
+                           const double* gcb, const double* eps, const double* sig, double* ge, double* gs,
+                           cudaStream_t st);
+
 // Incident beam (fdtd_incident.cu). The taper of incidentbeam.py:317-433
 // for a lateral grid of nx x ny cells and nt pulse bins: dfx = 1 / (nx dx),
 // dfy = 1 / (ny dx) (numpy.fft.fftfreq spacing), the incidence angles'

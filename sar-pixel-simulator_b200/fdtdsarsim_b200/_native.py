@@ -132,6 +132,7 @@ SIGNATURES = {
     'fdtd_near2far': [_P, _P, _P, _P, _I, _I, _I, _I, _D, _D, _P, _I, _P, _I, _D, _I, _P],
     'fdtd_grad_forward': [_P, _I],
     'fdtd_grad_backward': [_P, _P, _P, _I, _P, _P],
+    'fdtd_grad_backward_eps_sigma': [_P, _P, _P, _I, _P, _P, _P, _P],
     'fdtd_batch_create': [ctypes.POINTER(_P), _I, ctypes.POINTER(_P)],
     'fdtd_batch_destroy': [_P],
     'fdtd_batch_set_option': [_P, _I, _I],
@@ -363,20 +364,40 @@ class NativeSim:
         (fdtd_grad_forward)."""
         check(lib.fdtd_grad_forward(self.h, int(checkpoint_every)))
 
-    def grad_backward(self, dj_dre, dj_dim, nz_out):
-        """dJ/dCa, dJ/dCb of the first nz_out planes from dJ/d(Re, Im) of the
-        four upper-plane phasors, each (4, ny_ph, nx_ph) float64
-        (fdtd_grad_backward)."""
+    def _phasor_gradients(self, dj_dre, dj_dim):
         g = self.geom
         shape = (4, g.ny - 2 * g.npml, g.nx - 2 * g.npml)
         re = np.ascontiguousarray(dj_dre, dtype=np.float64)
         im = np.ascontiguousarray(dj_dim, dtype=np.float64)
         if re.shape != shape or im.shape != shape:
             raise ValueError(f'phasor gradients must have shape {shape}')
+        return re, im
+
+    def grad_backward(self, dj_dre, dj_dim, nz_out):
+        """dJ/dCa, dJ/dCb of the first nz_out planes from dJ/d(Re, Im) of the
+        four upper-plane phasors, each (4, ny_ph, nx_ph) float64
+        (fdtd_grad_backward)."""
+        g = self.geom
+        re, im = self._phasor_gradients(dj_dre, dj_dim)
         gca = np.empty((int(nz_out), g.ny, g.nx), np.float64)
         gcb = np.empty_like(gca)
         check(lib.fdtd_grad_backward(self.h, ptr(re), ptr(im), int(nz_out), ptr(gca), ptr(gcb)))
         return gca, gcb
+
+    def grad_backward_eps_sigma(self, dj_dre, dj_dim, eps_r, sigma):
+        """dJ/deps_r, dJ/dsigma of the material block (nz, ny, nx) whose
+        values are given (fdtd_grad_backward_eps_sigma); float64."""
+        g = self.geom
+        re, im = self._phasor_gradients(dj_dre, dj_dim)
+        e = np.ascontiguousarray(eps_r, dtype=np.float64)
+        s = np.ascontiguousarray(sigma, dtype=np.float64)
+        if e.shape != s.shape or e.ndim != 3 or e.shape[1:] != (g.ny, g.nx):
+            raise ValueError(f'eps/sigma must both be (nz_mat, {g.ny}, {g.nx})')
+        ge = np.empty(e.shape, np.float64)
+        gs = np.empty_like(ge)
+        check(lib.fdtd_grad_backward_eps_sigma(self.h, ptr(re), ptr(im), int(e.shape[0]), ptr(e), ptr(s),
+                                               ptr(ge), ptr(gs)))
+        return ge, gs
 
     def get_fields(self):
         return {c: self.get_field(c) for c in FIELD_NAMES}

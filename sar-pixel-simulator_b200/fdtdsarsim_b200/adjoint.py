@@ -25,7 +25,6 @@ import numpy as np
 
 from . import _native
 from .absorbers import packed_profiles
-from .materials import MaterialModel, compute_material_arrays
 from .parameters import ParameterCollection
 
 ETA0 = 376.730313668
@@ -133,12 +132,16 @@ class BackscatterGradient:
             params.inc_beam_params.frequency, pol)
 
     def _set_materials(self, eps_r, sigma):
-        g = self.params.geom_params
+        # Ca, Cb on the device, bit for bit those of compute_material_arrays
         dt = self.params.processing_params.datatype
-        model = MaterialModel(np.asarray(eps_r, dtype=dt), np.asarray(sigma, dtype=dt),
-                              g.cell_size)
-        ca, cb = compute_material_arrays(self.params, model)
-        self.sim.set_materials(ca, cb)
+        eps_r, sigma = np.asarray(eps_r, dtype=dt), np.asarray(sigma, dtype=dt)
+        if eps_r.shape != sigma.shape:
+            raise RuntimeError('Permittivity and conductivity arrays have different shapes')
+        g = self.params.geom_params
+        shape = (g.size_z_material, g.size_y, g.size_x)
+        if eps_r.shape != shape:
+            raise ValueError(f'material block must have shape {shape}, got {eps_r.shape}')
+        self.sim.set_materials_eps_sigma(eps_r, sigma)
 
     def _upper_phasors(self):
         return np.stack([self.sim.get_phasor(k).astype(np.complex128) for k in (4, 5, 6, 7)])
@@ -154,14 +157,12 @@ class BackscatterGradient:
     def value_and_grad(self, eps_r, sigma):
         """(P, dP/deps_r, dP/dsigma), the gradients with the material block's
         shape, in float64."""
-        g = self.params.geom_params
         self._set_materials(eps_r, sigma)
         self.sim.grad_forward(self.every)
         J, g_re, g_im = power_and_phasor_grad(self._upper_phasors(), self.a, self.b, self.sign)
-        nzm = g.size_z_material
-        gca, gcb = self.sim.grad_backward(g_re, g_im, nzm)
-        dca_de, dca_ds, dcb_de, dcb_ds = ca_cb_partials(eps_r, sigma, g.timestep, g.cell_size)
-        return J, gca * dca_de + gcb * dcb_de, gca * dca_ds + gcb * dcb_ds
+        # through ca_cb_partials, evaluated on the device
+        ge, gs = self.sim.grad_backward_eps_sigma(g_re, g_im, eps_r, sigma)
+        return J, ge, gs
 
     def close(self):
         self.sim.close()
