@@ -162,20 +162,60 @@ __global__ void k_adj_phasor_e(const __grid_constant__ State<T> s, Adj<T> a, int
 }
 
 // ---- vector form ------------------------------------------------------------
-// A thread owns four consecutive x cells of one row (x0 a multiple of 4;
-// the pitch is a multiple of 32 elements, so the four cells are one aligned
-// vector in every (.., pitch)-strided array, as in the forward step). z- and
-// y-face auxiliaries have coefficients uniform over the vector; x-face
-// auxiliaries ((z, y, npml) layout) run per cell.
+// A thread owns two consecutive x cells of one row (x0 even; the pitch is a
+// multiple of 32 elements, so the two are one aligned vector in every (..,
+// pitch)-strided array). z- and y-face auxiliaries have coefficients uniform
+// over the vector; x-face auxiliaries ((z, y, npml) layout) run per cell.
+//
+// Two cells, not the forward step's four: the kernels are bound by latency
+// (IPC 1 at 96 and 128 registers with four cells, 16 to 20 warps per SM),
+// and two cells take half the registers, 64 and 72. The backward half per
+// step with four and two cells, us: 55 x 133 x 133 cells float 82 and 72,
+// 81 x 231 x 229 381 and 308, 39 x 61 x 57 29 and 26, 55 x 133 x 133 double
+// 201 and 149 (one cell, 55 x 133 x 133 float: 75). Blocks per SM: 8 and 7
+// for float (2 to 3 us better than 10 and 8; no minimum: 8 us worse), 7 and
+// 6 for double (5 and 4: 156, none: 163).
+constexpr int kAdj = 2;
+
+template <class T>
+struct alignas(kAdj * sizeof(T)) AdjVec {
+  T v[kAdj];
+};
+
+template <class T>
+__device__ __forceinline__ void zero_adj(T (&d)[kAdj]) {
+#pragma unroll
+  for (int j = 0; j < kAdj; ++j) d[j] = T(0);
+}
+
+template <class T>
+__device__ __forceinline__ void ld_adj(T (&d)[kAdj], const T* p) {
+  if (!FDTD_CHECK_PTR(p, (int)sizeof(T) * kAdj)) {   // bounds-checked build only
+    zero_adj(d);
+    return;
+  }
+  const AdjVec<T> q = *reinterpret_cast<const AdjVec<T>*>(p);
+#pragma unroll
+  for (int j = 0; j < kAdj; ++j) d[j] = q.v[j];
+}
+
+template <class T>
+__device__ __forceinline__ void st_adj(T* p, const T (&d)[kAdj]) {
+  if (!FDTD_CHECK_PTR(p, (int)sizeof(T) * kAdj)) return;   // bounds-checked build only
+  AdjVec<T> q;
+#pragma unroll
+  for (int j = 0; j < kAdj; ++j) q.v[j] = d[j];
+  *reinterpret_cast<AdjVec<T>*>(p) = q;
+}
 
 // main-update ranges of the E components of the vector's cells
 template <class T>
-__device__ __forceinline__ void e_ranges(const State<T>& s, int z, int y, int x0, bool (&rx)[kVec],
-                                         bool (&ry)[kVec], bool (&rz)[kVec]) {
+__device__ __forceinline__ void e_ranges(const State<T>& s, int z, int y, int x0, bool (&rx)[kAdj],
+                                         bool (&ry)[kAdj], bool (&rz)[kAdj]) {
   const bool zi = z >= 1 && z < s.nz - 1, yi = y >= 1 && y < s.ny - 1;
   const bool zb = z >= 0 && z < s.nz - 1, yb = y >= 0 && y < s.ny - 1;
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     const int x = x0 + j;
     const bool xb = x < s.nx - 1, xi = x >= 1 && x < s.nx - 1;
     rx[j] = zi && yi && xb;
@@ -186,12 +226,12 @@ __device__ __forceinline__ void e_ranges(const State<T>& s, int z, int y, int x0
 
 // and of the H components
 template <class T>
-__device__ __forceinline__ void h_ranges(const State<T>& s, int z, int y, int x0, bool (&rx)[kVec],
-                                         bool (&ry)[kVec], bool (&rz)[kVec]) {
+__device__ __forceinline__ void h_ranges(const State<T>& s, int z, int y, int x0, bool (&rx)[kAdj],
+                                         bool (&ry)[kAdj], bool (&rz)[kAdj]) {
   const bool zi = z >= 1 && z < s.nz - 1, yi = y >= 1 && y < s.ny - 1;
   const bool zb = z >= 0 && z < s.nz - 1, yb = y >= 0 && y < s.ny - 1;
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     const int x = x0 + j;
     const bool xb = x < s.nx - 1, xi = x >= 1 && x < s.nx - 1;
     rx[j] = zb && yb && xi;
@@ -202,10 +242,10 @@ __device__ __forceinline__ void h_ranges(const State<T>& s, int z, int y, int x0
 
 // F = Cb lambda_E of one component where `r` holds
 template <class T>
-__device__ __forceinline__ void masked_prod(T (&f)[kVec], const T (&cb)[kVec], const T (&l)[kVec],
-                                            const bool (&r)[kVec]) {
+__device__ __forceinline__ void masked_prod(T (&f)[kAdj], const T (&cb)[kAdj], const T (&l)[kAdj],
+                                            const bool (&r)[kAdj]) {
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) f[j] = r[j] ? cb[j] * l[j] : T(0);
+  for (int j = 0; j < kAdj; ++j) f[j] = r[j] ? cb[j] * l[j] : T(0);
 }
 
 // E-face auxiliaries of plane zz (z faces) or row yy (y faces): c/dx times
@@ -214,19 +254,19 @@ __device__ __forceinline__ void masked_prod(T (&f)[kVec], const T (&cb)[kVec], c
 // z faces: t0 Exz (F = fx, sign -), t1 Eyz (fy, +).
 template <class T>
 __device__ __forceinline__ void e_zface(const State<T>& s, const Adj<T>& a, int zz, int y, int x0,
-                                        const T (&fx)[kVec], const T (&fy)[kVec], T (&t0)[kVec],
-                                        T (&t1)[kVec]) {
-  zero4(t0);
-  zero4(t1);
+                                        const T (&fx)[kAdj], const T (&fy)[kAdj], T (&t0)[kAdj],
+                                        T (&t1)[kAdj]) {
+  zero_adj(t0);
+  zero_adj(t1);
   int side, q;
   if (zz >= s.nz - 1 || y >= s.ny - 1 || !e_face(zz, s.nz, s.npml, side, q)) return;
   const long long k = kz(s, q, y, x0);
   const T c = s.prof[side ? CE_U : CE_D][q] * s.rdx;
-  T p0[kVec], p1[kVec];
-  ld4(p0, a.lps.z[side][0] + k);
-  ld4(p1, a.lps.z[side][1] + k);
+  T p0[kAdj], p1[kAdj];
+  ld_adj(p0, a.lps.z[side][0] + k);
+  ld_adj(p1, a.lps.z[side][1] + k);
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     if (x0 + j >= s.nx - 1) continue;
     t0[j] = c * (p0[j] - s.dx * fx[j]);
     t1[j] = c * (p1[j] + s.dx * fy[j]);
@@ -236,19 +276,19 @@ __device__ __forceinline__ void e_zface(const State<T>& s, const Adj<T>& a, int 
 // y faces: t0 Exy (F = fx, sign +), t1 Ezy (fz, -).
 template <class T>
 __device__ __forceinline__ void e_yface(const State<T>& s, const Adj<T>& a, int z, int yy, int x0,
-                                        const T (&fx)[kVec], const T (&fz)[kVec], T (&t0)[kVec],
-                                        T (&t1)[kVec]) {
-  zero4(t0);
-  zero4(t1);
+                                        const T (&fx)[kAdj], const T (&fz)[kAdj], T (&t0)[kAdj],
+                                        T (&t1)[kAdj]) {
+  zero_adj(t0);
+  zero_adj(t1);
   int side, q;
   if (z >= s.nz - 1 || yy >= s.ny - 1 || !e_face(yy, s.ny, s.npml, side, q)) return;
   const long long k = ky(s, z, q, x0);
   const T c = s.prof[side ? CE_U : CE_D][q] * s.rdx;
-  T p0[kVec], p1[kVec];
-  ld4(p0, a.lps.y[side][0] + k);
-  ld4(p1, a.lps.y[side][1] + k);
+  T p0[kAdj], p1[kAdj];
+  ld_adj(p0, a.lps.y[side][0] + k);
+  ld_adj(p1, a.lps.y[side][1] + k);
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     if (x0 + j >= s.nx - 1) continue;
     t0[j] = c * (p0[j] + s.dx * fx[j]);
     t1[j] = c * (p1[j] - s.dx * fz[j]);
@@ -259,19 +299,19 @@ __device__ __forceinline__ void e_yface(const State<T>& s, const Adj<T>& a, int 
 // z faces: t2 Hxz (lhx, +), t3 Hyz (lhy, -).
 template <class T>
 __device__ __forceinline__ void h_zface(const State<T>& s, const Adj<T>& a, int zz, int y, int x0,
-                                        const T (&lx)[kVec], const T (&ly)[kVec], T (&t2)[kVec],
-                                        T (&t3)[kVec]) {
-  zero4(t2);
-  zero4(t3);
+                                        const T (&lx)[kAdj], const T (&ly)[kAdj], T (&t2)[kAdj],
+                                        T (&t3)[kAdj]) {
+  zero_adj(t2);
+  zero_adj(t3);
   int side, q;
   if (zz < 0 || zz >= s.nz - 1 || y >= s.ny - 1 || !h_face(zz, s.nz, s.npml, side, q)) return;
   const long long k = kz(s, q, y, x0);
   const T c = s.prof[side ? CH_U : CH_D][q] * s.rdx;
-  T p2[kVec], p3[kVec];
-  ld4(p2, a.lps.z[side][2] + k);
-  ld4(p3, a.lps.z[side][3] + k);
+  T p2[kAdj], p3[kAdj];
+  ld_adj(p2, a.lps.z[side][2] + k);
+  ld_adj(p3, a.lps.z[side][3] + k);
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     if (x0 + j >= s.nx - 1) continue;
     t2[j] = c * (p2[j] + s.dtm0 * lx[j]);
     t3[j] = c * (p3[j] - s.dtm0 * ly[j]);
@@ -281,19 +321,19 @@ __device__ __forceinline__ void h_zface(const State<T>& s, const Adj<T>& a, int 
 // y faces: t2 Hxy (lhx, -), t3 Hzy (lhz, +).
 template <class T>
 __device__ __forceinline__ void h_yface(const State<T>& s, const Adj<T>& a, int z, int yy, int x0,
-                                        const T (&lx)[kVec], const T (&lz)[kVec], T (&t2)[kVec],
-                                        T (&t3)[kVec]) {
-  zero4(t2);
-  zero4(t3);
+                                        const T (&lx)[kAdj], const T (&lz)[kAdj], T (&t2)[kAdj],
+                                        T (&t3)[kAdj]) {
+  zero_adj(t2);
+  zero_adj(t3);
   int side, q;
   if (yy < 0 || z >= s.nz - 1 || yy >= s.ny - 1 || !h_face(yy, s.ny, s.npml, side, q)) return;
   const long long k = ky(s, z, q, x0);
   const T c = s.prof[side ? CH_U : CH_D][q] * s.rdx;
-  T p2[kVec], p3[kVec];
-  ld4(p2, a.lps.y[side][2] + k);
-  ld4(p3, a.lps.y[side][3] + k);
+  T p2[kAdj], p3[kAdj];
+  ld_adj(p2, a.lps.y[side][2] + k);
+  ld_adj(p3, a.lps.y[side][3] + k);
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     if (x0 + j >= s.nx - 1) continue;
     t2[j] = c * (p2[j] - s.dtm0 * lx[j]);
     t3[j] = c * (p3[j] + s.dtm0 * lz[j]);
@@ -304,29 +344,29 @@ __device__ __forceinline__ void h_yface(const State<T>& s, const Adj<T>& a, int 
 // lambda_psi = bh (lambda_psi + sign dtm0 lambda_H) on every H face.
 template <class T>
 __device__ __forceinline__ void h_own_vec(const State<T>& s, const Adj<T>& a, int z, int y, int x0,
-                                          const T (&lhx)[kVec], const T (&lhy)[kVec],
-                                          const T (&lhz)[kVec]) {
+                                          const T (&lhx)[kAdj], const T (&lhy)[kAdj],
+                                          const T (&lhz)[kAdj]) {
   const int nx = s.nx, ny = s.ny, nz = s.nz, m = s.npml;
   if (z >= nz - 1 || y >= ny - 1) return;
   int side, q;
   if (h_face(z, nz, m, side, q)) {
     const long long k = kz(s, q, y, x0);
     const T b = s.prof[side ? BH_U : BH_D][q];
-    T p2[kVec], p3[kVec];
-    ld4(p2, a.lps.z[side][2] + k);
-    ld4(p3, a.lps.z[side][3] + k);
+    T p2[kAdj], p3[kAdj];
+    ld_adj(p2, a.lps.z[side][2] + k);
+    ld_adj(p3, a.lps.z[side][3] + k);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       if (x0 + j >= nx - 1) continue;
       p3[j] = b * (p3[j] - s.dtm0 * lhy[j]);
       p2[j] = b * (p2[j] + s.dtm0 * lhx[j]);
     }
-    st4(a.lps.z[side][2] + k, p2);
-    st4(a.lps.z[side][3] + k, p3);
+    st_adj(a.lps.z[side][2] + k, p2);
+    st_adj(a.lps.z[side][3] + k, p3);
   }
-  if (x0 < m - 1 || x0 + kVec - 1 >= nx - m) {
+  if (x0 < m - 1 || x0 + kAdj - 1 >= nx - m) {
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       const int x = x0 + j;
       if (x >= nx - 1 || !h_face(x, nx, m, side, q)) continue;
       const long long k = kx(s, z, y, side, q);
@@ -340,17 +380,17 @@ __device__ __forceinline__ void h_own_vec(const State<T>& s, const Adj<T>& a, in
   if (h_face(y, ny, m, side, q)) {
     const long long k = ky(s, z, q, x0);
     const T b = s.prof[side ? BH_U : BH_D][q];
-    T p2[kVec], p3[kVec];
-    ld4(p2, a.lps.y[side][2] + k);
-    ld4(p3, a.lps.y[side][3] + k);
+    T p2[kAdj], p3[kAdj];
+    ld_adj(p2, a.lps.y[side][2] + k);
+    ld_adj(p3, a.lps.y[side][3] + k);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       if (x0 + j >= nx - 1) continue;
       p2[j] = b * (p2[j] - s.dtm0 * lhx[j]);
       p3[j] = b * (p3[j] + s.dtm0 * lhz[j]);
     }
-    st4(a.lps.y[side][2] + k, p2);
-    st4(a.lps.y[side][3] + k, p3);
+    st_adj(a.lps.y[side][2] + k, p2);
+    st_adj(a.lps.y[side][3] + k, p3);
   }
 }
 
@@ -361,91 +401,110 @@ __device__ __forceinline__ void h_own_vec(const State<T>& s, const Adj<T>& a, in
 // every neighbour it reads lie away from every CPML face and domain edge.
 template <class T, bool kFast>
 __device__ __forceinline__ void e_to_h_vec(const State<T>& s, const Adj<T>& a, int z, int y, int x0,
-                                           T (&dhx)[kVec], T (&dhy)[kVec], T (&dhz)[kVec]) {
+                                           T (&dhx)[kAdj], T (&dhy)[kAdj], T (&dhz)[kAdj]) {
   const int nx = s.nx, ny = s.ny, nz = s.nz, m = s.npml;
   const long long P = s.plane, W = s.pitch, i = idx(s, z, y, x0);
-  T cb[kVec], l0[kVec], l1[kVec], l2[kVec];
-  T fx[kVec], fy[kVec], fz[kVec];       // cell
-  T fxz[kVec], fyz[kVec];               // z + 1
-  T fxy[kVec], fzy[kVec];               // y + 1
-  T fyn = T(0), fzn = T(0);             // x0 + 4
-  ld4(cb, s.cb + i);
-  ld4(l0, a.lex + i);
-  ld4(l1, a.ley + i);
-  ld4(l2, a.lez + i);
+  T cb[kAdj], l0[kAdj], l1[kAdj], l2[kAdj];
+  T fx[kAdj], fy[kAdj], fz[kAdj];       // cell
+  ld_adj(cb, s.cb + i);
+  ld_adj(l0, a.lex + i);
+  ld_adj(l1, a.ley + i);
+  ld_adj(l2, a.lez + i);
   if constexpr (kFast) {
+    // The neighbours' products go into the differences unrounded, but for
+    // the x neighbour inside an aligned group of four cells, whose product
+    // is rounded as that cell's own: written out, so that the rounding of a
+    // cell depends on neither kAdj nor the compiler's contraction.
+    using M = R<T>;
+    T yz[kAdj], zy[kAdj], zx[kAdj], xz[kAdj], xy[kAdj], yx[kAdj];
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-      fx[j] = cb[j] * l0[j];
-      fy[j] = cb[j] * l1[j];
-      fz[j] = cb[j] * l2[j];
+    for (int j = 0; j < kAdj; ++j) {
+      fx[j] = M::mul(cb[j], l0[j]);
+      fy[j] = M::mul(cb[j], l1[j]);
+      fz[j] = M::mul(cb[j], l2[j]);
     }
-    ld4(cb, s.cb + i + P);
-    ld4(l0, a.lex + i + P);
-    ld4(l1, a.ley + i + P);
+    ld_adj(cb, s.cb + i + P);
+    ld_adj(l0, a.lex + i + P);
+    ld_adj(l1, a.ley + i + P);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-      fxz[j] = cb[j] * l0[j];
-      fyz[j] = cb[j] * l1[j];
+    for (int j = 0; j < kAdj; ++j) {
+      xz[j] = M::fma(-cb[j], l0[j], fx[j]);
+      yz[j] = M::fma(-cb[j], l1[j], fy[j]);
     }
-    ld4(cb, s.cb + i + W);
-    ld4(l0, a.lex + i + W);
-    ld4(l2, a.lez + i + W);
+    ld_adj(cb, s.cb + i + W);
+    ld_adj(l0, a.lex + i + W);
+    ld_adj(l2, a.lez + i + W);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-      fxy[j] = cb[j] * l0[j];
-      fzy[j] = cb[j] * l2[j];
+    for (int j = 0; j < kAdj; ++j) {
+      xy[j] = M::fma(-cb[j], l0[j], fx[j]);
+      zy[j] = M::fma(-cb[j], l2[j], fz[j]);
     }
-    const T cbn = s.cb[i + kVec];
-    fyn = cbn * a.ley[i + kVec];
-    fzn = cbn * a.lez[i + kVec];
+    const T cbn = s.cb[i + kAdj], yn = a.ley[i + kAdj], zn = a.lez[i + kAdj];
+    const bool group = ((x0 + kAdj) & 3) == 0;   // x0 + kAdj starts the next group
+#pragma unroll
+    for (int j = 0; j < kAdj; ++j) {
+      if (j + 1 < kAdj) {
+        yx[j] = M::sub(fy[j], fy[j + 1 < kAdj ? j + 1 : j]);
+        zx[j] = M::sub(fz[j], fz[j + 1 < kAdj ? j + 1 : j]);
+      } else {
+        yx[j] = group ? M::fma(-cbn, yn, fy[j]) : M::sub(fy[j], M::mul(cbn, yn));
+        zx[j] = group ? M::fma(-cbn, zn, fz[j]) : M::sub(fz[j], M::mul(cbn, zn));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kAdj; ++j) {
+      dhx[j] = M::sub(yz[j], zy[j]);
+      dhy[j] = M::sub(zx[j], xz[j]);
+      dhz[j] = M::sub(xy[j], yx[j]);
+    }
   } else {
-    bool rx[kVec], ry[kVec], rz[kVec];
+    T fxz[kAdj], fyz[kAdj];             // z + 1
+    T fxy[kAdj], fzy[kAdj];             // y + 1
+    T fyn = T(0), fzn = T(0);           // x0 + kAdj
+    bool rx[kAdj], ry[kAdj], rz[kAdj];
     e_ranges(s, z, y, x0, rx, ry, rz);
     masked_prod(fx, cb, l0, rx);
     masked_prod(fy, cb, l1, ry);
     masked_prod(fz, cb, l2, rz);
-    zero4(fxz);
-    zero4(fyz);
+    zero_adj(fxz);
+    zero_adj(fyz);
     if (z + 1 < nz - 1) {
       e_ranges(s, z + 1, y, x0, rx, ry, rz);
-      ld4(cb, s.cb + i + P);
-      ld4(l0, a.lex + i + P);
-      ld4(l1, a.ley + i + P);
+      ld_adj(cb, s.cb + i + P);
+      ld_adj(l0, a.lex + i + P);
+      ld_adj(l1, a.ley + i + P);
       masked_prod(fxz, cb, l0, rx);
       masked_prod(fyz, cb, l1, ry);
     }
-    zero4(fxy);
-    zero4(fzy);
+    zero_adj(fxy);
+    zero_adj(fzy);
     if (y + 1 < ny - 1) {
       e_ranges(s, z, y + 1, x0, rx, ry, rz);
-      ld4(cb, s.cb + i + W);
-      ld4(l0, a.lex + i + W);
-      ld4(l2, a.lez + i + W);
+      ld_adj(cb, s.cb + i + W);
+      ld_adj(l0, a.lex + i + W);
+      ld_adj(l2, a.lez + i + W);
       masked_prod(fxy, cb, l0, rx);
       masked_prod(fzy, cb, l2, rz);
     }
-    if (x0 + kVec < nx - 1) {   // the cell x0 + 4 is inside the x ranges
-      const T cbn = s.cb[i + kVec];
-      if (z >= 1 && z < nz - 1 && y < ny - 1) fyn = cbn * a.ley[i + kVec];
-      if (z < nz - 1 && y >= 1 && y < ny - 1) fzn = cbn * a.lez[i + kVec];
+    if (x0 + kAdj < nx - 1) {   // the cell x0 + kAdj is inside the x ranges
+      const T cbn = s.cb[i + kAdj];
+      if (z >= 1 && z < nz - 1 && y < ny - 1) fyn = cbn * a.ley[i + kAdj];
+      if (z < nz - 1 && y >= 1 && y < ny - 1) fzn = cbn * a.lez[i + kAdj];
     }
-  }
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
-    const T fy_x = j + 1 < kVec ? fy[j + 1 < kVec ? j + 1 : j] : fyn;
-    const T fz_x = j + 1 < kVec ? fz[j + 1 < kVec ? j + 1 : j] : fzn;
-    dhx[j] = (fy[j] - fyz[j]) - (fz[j] - fzy[j]);
-    dhy[j] = (fz[j] - fz_x) - (fx[j] - fxz[j]);
-    dhz[j] = (fx[j] - fxy[j]) - (fy[j] - fy_x);
-  }
-  if constexpr (!kFast) {
-    T t0[kVec], t1[kVec], u0[kVec], u1[kVec];
+    for (int j = 0; j < kAdj; ++j) {
+      const T fy_x = j + 1 < kAdj ? fy[j + 1 < kAdj ? j + 1 : j] : fyn;
+      const T fz_x = j + 1 < kAdj ? fz[j + 1 < kAdj ? j + 1 : j] : fzn;
+      dhx[j] = (fy[j] - fyz[j]) - (fz[j] - fzy[j]);
+      dhy[j] = (fz[j] - fz_x) - (fx[j] - fxz[j]);
+      dhz[j] = (fx[j] - fxy[j]) - (fy[j] - fy_x);
+    }
+    T t0[kAdj], t1[kAdj], u0[kAdj], u1[kAdj];
     // z faces of the cell and of z + 1: Eyz reads hx(c) - hx(c - z), Exz hy
     e_zface(s, a, z, y, x0, fx, fy, t0, t1);
     e_zface(s, a, z + 1, y, x0, fxz, fyz, u0, u1);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       dhx[j] += t1[j] - u1[j];
       dhy[j] += t0[j] - u0[j];
     }
@@ -453,18 +512,18 @@ __device__ __forceinline__ void e_to_h_vec(const State<T>& s, const Adj<T>& a, i
     e_yface(s, a, z, y, x0, fx, fz, t0, t1);
     e_yface(s, a, z, y + 1, x0, fxy, fzy, u0, u1);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       dhz[j] += t0[j] - u0[j];
       dhx[j] += t1[j] - u1[j];
     }
-    // x faces of x0 .. x0 + 4: Ezx reads hy(c) - hy(c - x), Eyx hz
-    if (x0 < m || x0 + kVec >= nx - m) {
-      T xt0[kVec + 1], xt1[kVec + 1];
+    // x faces of x0 .. x0 + kAdj: Ezx reads hy(c) - hy(c - x), Eyx hz
+    if (x0 < m || x0 + kAdj >= nx - m) {
+      T xt0[kAdj + 1], xt1[kAdj + 1];
 #pragma unroll
-      for (int p = 0; p <= kVec; ++p) {
+      for (int p = 0; p <= kAdj; ++p) {
         const int xx = x0 + p;
-        const T fyv = p < kVec ? fy[p < kVec ? p : 0] : fyn;
-        const T fzv = p < kVec ? fz[p < kVec ? p : 0] : fzn;
+        const T fyv = p < kAdj ? fy[p < kAdj ? p : 0] : fyn;
+        const T fzv = p < kAdj ? fz[p < kAdj ? p : 0] : fzn;
         xt0[p] = T(0);
         xt1[p] = T(0);
         int side, q;
@@ -476,7 +535,7 @@ __device__ __forceinline__ void e_to_h_vec(const State<T>& s, const Adj<T>& a, i
         }
       }
 #pragma unroll
-      for (int j = 0; j < kVec; ++j) {
+      for (int j = 0; j < kAdj; ++j) {
         dhy[j] += xt1[j] - xt1[j + 1];
         dhz[j] += xt0[j] - xt0[j + 1];
       }
@@ -489,62 +548,62 @@ __device__ __forceinline__ void e_to_h_vec(const State<T>& s, const Adj<T>& a, i
 // H^{n+1/2}, s.ps the auxiliaries after the step.
 template <class T, bool kFast>
 __device__ __forceinline__ void e_own_vec(const State<T>& s, const Adj<T>& a, int z, int y, int x0,
-                                          T (&ox)[kVec], T (&oy)[kVec], T (&oz)[kVec]) {
+                                          T (&ox)[kAdj], T (&oy)[kAdj], T (&oz)[kAdj]) {
   const int nx = s.nx, ny = s.ny, nz = s.nz, m = s.npml;
   const long long P = s.plane, W = s.pitch, i = idx(s, z, y, x0);
-  T lx[kVec], ly[kVec], lz[kVec], ca[kVec], cb[kVec];
-  ld4(lx, a.lex + i);
-  ld4(ly, a.ley + i);
-  ld4(lz, a.lez + i);
-  ld4(ca, s.ca + i);
-  ld4(cb, s.cb + i);
-  bool rx[kVec], ry[kVec], rz[kVec];
+  T lx[kAdj], ly[kAdj], lz[kAdj], ca[kAdj], cb[kAdj];
+  ld_adj(lx, a.lex + i);
+  ld_adj(ly, a.ley + i);
+  ld_adj(lz, a.lez + i);
+  ld_adj(ca, s.ca + i);
+  ld_adj(cb, s.cb + i);
+  bool rx[kAdj], ry[kAdj], rz[kAdj];
   if constexpr (kFast) {
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) rx[j] = ry[j] = rz[j] = true;
+    for (int j = 0; j < kAdj; ++j) rx[j] = ry[j] = rz[j] = true;
   } else {
     e_ranges(s, z, y, x0, rx, ry, rz);
   }
   const bool grad = z < a.nz_grad;   // gradients only over the requested planes
-  double gca[kVec], gcb[kVec];
+  double gca[kAdj], gcb[kAdj];
   if (grad) {
-    T e[kVec], h0[kVec], h1[kVec], h2[kVec], hn0[kVec], hn1[kVec];
-    ld4(e, s.iex + i);
+    T e[kAdj], h0[kAdj], h1[kAdj], h2[kAdj], hn0[kAdj], hn1[kAdj];
+    ld_adj(e, s.iex + i);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) gca[j] = rx[j] ? (double)lx[j] * (double)e[j] : 0.0;
-    ld4(e, s.iey + i);
+    for (int j = 0; j < kAdj; ++j) gca[j] = rx[j] ? (double)lx[j] * (double)e[j] : 0.0;
+    ld_adj(e, s.iey + i);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) gca[j] += ry[j] ? (double)ly[j] * (double)e[j] : 0.0;
-    ld4(e, s.iez + i);
+    for (int j = 0; j < kAdj; ++j) gca[j] += ry[j] ? (double)ly[j] * (double)e[j] : 0.0;
+    ld_adj(e, s.iez + i);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) gca[j] += rz[j] ? (double)lz[j] * (double)e[j] : 0.0;
-    ld4(h0, s.ihx + i);
-    ld4(h1, s.ihy + i);
-    ld4(h2, s.ihz + i);
+    for (int j = 0; j < kAdj; ++j) gca[j] += rz[j] ? (double)lz[j] * (double)e[j] : 0.0;
+    ld_adj(h0, s.ihx + i);
+    ld_adj(h1, s.ihy + i);
+    ld_adj(h2, s.ihz + i);
     // ex: (hz - hz(y-1)) - (hy - hy(z-1))
     if (kFast || (z >= 1 && y >= 1)) {
-      ld4(hn0, s.ihz + i - W);
-      ld4(hn1, s.ihy + i - P);
+      ld_adj(hn0, s.ihz + i - W);
+      ld_adj(hn1, s.ihy + i - P);
     } else {
-      zero4(hn0);
-      zero4(hn1);
+      zero_adj(hn0);
+      zero_adj(hn1);
     }
 #pragma unroll
-    for (int j = 0; j < kVec; ++j)
+    for (int j = 0; j < kAdj; ++j)
       gcb[j] = rx[j] ? (double)lx[j] * (double)((h2[j] - hn0[j]) - (h1[j] - hn1[j])) : 0.0;
     // ey: (hx - hx(z-1)) - (hz - hz(x-1))
     const T hzp = (kFast || (x0 >= 1 && z >= 1)) ? s.ihz[i - 1] : T(0);
-    if (kFast || z >= 1) ld4(hn0, s.ihx + i - P); else zero4(hn0);
+    if (kFast || z >= 1) ld_adj(hn0, s.ihx + i - P); else zero_adj(hn0);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       const T hz_x = j > 0 ? h2[j > 0 ? j - 1 : 0] : hzp;
       gcb[j] += ry[j] ? (double)ly[j] * (double)((h0[j] - hn0[j]) - (h2[j] - hz_x)) : 0.0;
     }
     // ez: (hy - hy(x-1)) - (hx - hx(y-1))
     const T hyp = (kFast || (x0 >= 1 && y >= 1)) ? s.ihy[i - 1] : T(0);
-    if (kFast || y >= 1) ld4(hn0, s.ihx + i - W); else zero4(hn0);
+    if (kFast || y >= 1) ld_adj(hn0, s.ihx + i - W); else zero_adj(hn0);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       const T hy_x = j > 0 ? h1[j > 0 ? j - 1 : 0] : hyp;
       gcb[j] += rz[j] ? (double)lz[j] * (double)((h1[j] - hy_x) - (h0[j] - hn0[j])) : 0.0;
     }
@@ -556,26 +615,26 @@ __device__ __forceinline__ void e_own_vec(const State<T>& s, const Adj<T>& a, in
       if (e_face(z, nz, m, side, q)) {
         const long long k = kz(s, q, y, x0);
         const T b = s.prof[side ? BE_U : BE_D][q];
-        T p0[kVec], p1[kVec], s0[kVec], s1[kVec];
-        ld4(p0, a.lps.z[side][0] + k);
-        ld4(p1, a.lps.z[side][1] + k);
+        T p0[kAdj], p1[kAdj], s0[kAdj], s1[kAdj];
+        ld_adj(p0, a.lps.z[side][0] + k);
+        ld_adj(p1, a.lps.z[side][1] + k);
         if (grad) {
-          ld4(s0, s.ps.z[side][0] + k);
-          ld4(s1, s.ps.z[side][1] + k);
+          ld_adj(s0, s.ps.z[side][0] + k);
+          ld_adj(s1, s.ps.z[side][1] + k);
         }
 #pragma unroll
-        for (int j = 0; j < kVec; ++j) {
+        for (int j = 0; j < kAdj; ++j) {
           if (x0 + j >= nx - 1) continue;
           if (grad) gcb[j] += (double)dx * ((double)s1[j] * ly[j] - (double)s0[j] * lx[j]);
           p1[j] = b * (p1[j] + cb[j] * dx * ly[j]);
           p0[j] = b * (p0[j] - cb[j] * dx * lx[j]);
         }
-        st4(a.lps.z[side][0] + k, p0);
-        st4(a.lps.z[side][1] + k, p1);
+        st_adj(a.lps.z[side][0] + k, p0);
+        st_adj(a.lps.z[side][1] + k, p1);
       }
-      if (x0 < m || x0 + kVec - 1 >= nx - m) {
+      if (x0 < m || x0 + kAdj - 1 >= nx - m) {
 #pragma unroll
-        for (int j = 0; j < kVec; ++j) {
+        for (int j = 0; j < kAdj; ++j) {
           const int x = x0 + j;
           if (x >= nx - 1 || !e_face(x, nx, m, side, q)) continue;
           const long long k = kx(s, z, y, side, q);
@@ -591,35 +650,35 @@ __device__ __forceinline__ void e_own_vec(const State<T>& s, const Adj<T>& a, in
       if (e_face(y, ny, m, side, q)) {
         const long long k = ky(s, z, q, x0);
         const T b = s.prof[side ? BE_U : BE_D][q];
-        T p0[kVec], p1[kVec], s0[kVec], s1[kVec];
-        ld4(p0, a.lps.y[side][0] + k);
-        ld4(p1, a.lps.y[side][1] + k);
+        T p0[kAdj], p1[kAdj], s0[kAdj], s1[kAdj];
+        ld_adj(p0, a.lps.y[side][0] + k);
+        ld_adj(p1, a.lps.y[side][1] + k);
         if (grad) {
-          ld4(s0, s.ps.y[side][0] + k);
-          ld4(s1, s.ps.y[side][1] + k);
+          ld_adj(s0, s.ps.y[side][0] + k);
+          ld_adj(s1, s.ps.y[side][1] + k);
         }
 #pragma unroll
-        for (int j = 0; j < kVec; ++j) {
+        for (int j = 0; j < kAdj; ++j) {
           if (x0 + j >= nx - 1) continue;
           if (grad) gcb[j] += (double)dx * ((double)s0[j] * lx[j] - (double)s1[j] * lz[j]);
           p0[j] = b * (p0[j] + cb[j] * dx * lx[j]);
           p1[j] = b * (p1[j] - cb[j] * dx * lz[j]);
         }
-        st4(a.lps.y[side][0] + k, p0);
-        st4(a.lps.y[side][1] + k, p1);
+        st_adj(a.lps.y[side][0] + k, p0);
+        st_adj(a.lps.y[side][1] + k, p1);
       }
     }
   }
   if (grad) {
-    double g[kVec];
-    ld4(g, a.gca + i);
+    double g[kAdj];
+    ld_adj(g, a.gca + i);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) g[j] += gca[j];
-    st4(a.gca + i, g);
-    ld4(g, a.gcb + i);
+    for (int j = 0; j < kAdj; ++j) g[j] += gca[j];
+    st_adj(a.gca + i, g);
+    ld_adj(g, a.gcb + i);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) g[j] += gcb[j];
-    st4(a.gcb + i, g);
+    for (int j = 0; j < kAdj; ++j) g[j] += gcb[j];
+    st_adj(a.gcb + i, g);
   }
   // A component outside its main-update range is updated in the forward
   // step only by CPML corrections and injection terms that read other such
@@ -633,7 +692,7 @@ __device__ __forceinline__ void e_own_vec(const State<T>& s, const Adj<T>& a, in
   // sweep finite. Every reader below relies on that: adjoint fields are
   // exactly zero outside their update ranges.
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     ox[j] = rx[j] ? ca[j] * lx[j] : T(0);
     oy[j] = ry[j] ? ca[j] * ly[j] : T(0);
     oz[j] = rz[j] ? ca[j] * lz[j] : T(0);
@@ -646,28 +705,28 @@ __device__ __forceinline__ void e_own_vec(const State<T>& s, const Adj<T>& a, in
 // auxiliaries of the cell and of those neighbours.
 template <class T, bool kFast>
 __device__ __forceinline__ void h_to_e_vec(const State<T>& s, const Adj<T>& a, int z, int y, int x0,
-                                           T (&dex)[kVec], T (&dey)[kVec], T (&dez)[kVec]) {
+                                           T (&dex)[kAdj], T (&dey)[kAdj], T (&dez)[kAdj]) {
   const int nx = s.nx, ny = s.ny, nz = s.nz, m = s.npml;
   const long long P = s.plane, W = s.pitch, i = idx(s, z, y, x0);
-  T hx[kVec], hy[kVec], hz[kVec];       // lambda_H of the cell
-  T hxz[kVec], hyz[kVec];               // z - 1
-  T hxy[kVec], hzy[kVec];               // y - 1
-  ld4(hx, a.lhx + i);
-  ld4(hy, a.lhy + i);
-  ld4(hz, a.lhz + i);
+  T hx[kAdj], hy[kAdj], hz[kAdj];       // lambda_H of the cell
+  T hxz[kAdj], hyz[kAdj];               // z - 1
+  T hxy[kAdj], hzy[kAdj];               // y - 1
+  ld_adj(hx, a.lhx + i);
+  ld_adj(hy, a.lhy + i);
+  ld_adj(hz, a.lhz + i);
   if (kFast || z >= 1) {
-    ld4(hxz, a.lhx + i - P);
-    ld4(hyz, a.lhy + i - P);
+    ld_adj(hxz, a.lhx + i - P);
+    ld_adj(hyz, a.lhy + i - P);
   } else {
-    zero4(hxz);
-    zero4(hyz);
+    zero_adj(hxz);
+    zero_adj(hyz);
   }
   if (kFast || y >= 1) {
-    ld4(hxy, a.lhx + i - W);
-    ld4(hzy, a.lhz + i - W);
+    ld_adj(hxy, a.lhx + i - W);
+    ld_adj(hzy, a.lhz + i - W);
   } else {
-    zero4(hxy);
-    zero4(hzy);
+    zero_adj(hxy);
+    zero_adj(hzy);
   }
   T hyp = T(0), hzp = T(0);             // x0 - 1
   if (kFast || x0 >= 1) {
@@ -676,7 +735,7 @@ __device__ __forceinline__ void h_to_e_vec(const State<T>& s, const Adj<T>& a, i
   }
   const T db = s.db;
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     const T hy_x = j > 0 ? hy[j > 0 ? j - 1 : 0] : hyp;
     const T hz_x = j > 0 ? hz[j > 0 ? j - 1 : 0] : hzp;
     dex[j] = db * ((hy[j] - hyz[j]) - (hz[j] - hzy[j]));
@@ -684,12 +743,12 @@ __device__ __forceinline__ void h_to_e_vec(const State<T>& s, const Adj<T>& a, i
     dez[j] = db * ((hx[j] - hxy[j]) - (hy[j] - hy_x));
   }
   if constexpr (!kFast) {
-    T t2[kVec], t3[kVec], u2[kVec], u3[kVec];
+    T t2[kAdj], t3[kAdj], u2[kAdj], u3[kAdj];
     // z faces of z - 1 and of the cell: Hyz reads ex(c + z) - ex(c), Hxz ey
     h_zface(s, a, z - 1, y, x0, hxz, hyz, t2, t3);
     h_zface(s, a, z, y, x0, hx, hy, u2, u3);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       dex[j] += t3[j] - u3[j];
       dey[j] += t2[j] - u2[j];
     }
@@ -697,15 +756,15 @@ __device__ __forceinline__ void h_to_e_vec(const State<T>& s, const Adj<T>& a, i
     h_yface(s, a, z, y - 1, x0, hxy, hzy, t2, t3);
     h_yface(s, a, z, y, x0, hx, hz, u2, u3);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       dez[j] += t2[j] - u2[j];
       dex[j] += t3[j] - u3[j];
     }
-    // x faces of x0 - 1 .. x0 + 3: Hzx reads ey(c + x) - ey(c), Hyx ez
-    if (x0 < m || x0 + kVec - 1 >= nx - m) {
-      T xt2[kVec + 1], xt3[kVec + 1];
+    // x faces of x0 - 1 .. x0 + kAdj - 1: Hzx reads ey(c + x) - ey(c), Hyx ez
+    if (x0 < m || x0 + kAdj - 1 >= nx - m) {
+      T xt2[kAdj + 1], xt3[kAdj + 1];
 #pragma unroll
-      for (int p = 0; p <= kVec; ++p) {
+      for (int p = 0; p <= kAdj; ++p) {
         const int xx = x0 - 1 + p;
         const T lyv = p > 0 ? hy[p > 0 ? p - 1 : 0] : hyp;
         const T lzv = p > 0 ? hz[p > 0 ? p - 1 : 0] : hzp;
@@ -720,7 +779,7 @@ __device__ __forceinline__ void h_to_e_vec(const State<T>& s, const Adj<T>& a, i
         }
       }
 #pragma unroll
-      for (int j = 0; j < kVec; ++j) {
+      for (int j = 0; j < kAdj; ++j) {
         dey[j] += xt3[j] - xt3[j + 1];
         dez[j] += xt2[j] - xt2[j + 1];
       }
@@ -729,11 +788,11 @@ __device__ __forceinline__ void h_to_e_vec(const State<T>& s, const Adj<T>& a, i
 }
 
 // ---- the two kernels of one backward step ------------------------------------
-// Blocks of (lanes, 128 / lanes) threads, each thread four x cells; grid
+// Blocks of (lanes, 128 / lanes) threads, each thread kAdj x cells; grid
 // (x tiles, y tiles, nz).
 template <class T>
 __device__ __forceinline__ bool vec_cell(const State<T>& s, int& z, int& y, int& x0) {
-  x0 = kVec * (blockIdx.x * blockDim.x + threadIdx.x);
+  x0 = kAdj * (blockIdx.x * blockDim.x + threadIdx.x);
   y = blockIdx.y * blockDim.y + threadIdx.y;
   z = blockIdx.z;
   return x0 < s.nx && y < s.ny;
@@ -743,20 +802,22 @@ __device__ __forceinline__ bool vec_cell(const State<T>& s, int& z, int& y, int&
 // first backward step), then lambda_H += (E step)^T lambda_E + the H phasor
 // source of step n.
 template <class T>
-__global__ void __launch_bounds__(128) k_adj_k1(const __grid_constant__ State<T> s, Adj<T> a, int t,
-                                                int first) {
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 7)
+    k_adj_k1(const __grid_constant__ State<T> s, Adj<T> a, int t, int first) {
   int z, y, x0;
   if (!vec_cell(s, z, y, x0)) return;
   const int m = s.npml;
   const long long i = idx(s, z, y, x0);
-  T lhx[kVec], lhy[kVec], lhz[kVec], dhx[kVec], dhy[kVec], dhz[kVec];
-  ld4(lhx, a.lhx + i);
-  ld4(lhy, a.lhy + i);
-  ld4(lhz, a.lhz + i);
-  if (z >= m && z < s.nz - m - 1 && y >= m && y < s.ny - m - 1 && x0 >= m &&
-      x0 + kVec < s.nx - m) {
+  T lhx[kAdj], lhy[kAdj], lhz[kAdj], dhx[kAdj], dhy[kAdj], dhz[kAdj];
+  ld_adj(lhx, a.lhx + i);
+  ld_adj(lhy, a.lhy + i);
+  ld_adj(lhz, a.lhz + i);
+  const int xg = x0 & ~3;
+  if (z >= m && z < s.nz - m - 1 && y >= m && y < s.ny - m - 1 && xg >= m && xg + 4 < s.nx - m) {
     // no H face at the vector, no E face or domain edge at it or its +x,
-    // +y, +z neighbours
+    // +y, +z neighbours. The line is drawn for the aligned four cells: the
+    // general form rounds every product, the fast one does not, so the line
+    // decides a cell's last bit, which kAdj must not.
     e_to_h_vec<T, true>(s, a, z, y, x0, dhx, dhy, dhz);
   } else {
     if (!first) h_own_vec(s, a, z, y, x0, lhx, lhy, lhz);
@@ -765,40 +826,41 @@ __global__ void __launch_bounds__(128) k_adj_k1(const __grid_constant__ State<T>
   const int pz = s.nz - m - 1;
   if (z == pz || z == pz - 1) {
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       T phx, phy;
       phasor_h_src(s, a, t, z, y, x0 + j, phx, phy);
       dhx[j] += phx;
       dhy[j] += phy;
     }
   }
-  bool rx[kVec], ry[kVec], rz[kVec];
+  bool rx[kAdj], ry[kAdj], rz[kAdj];
   h_ranges(s, z, y, x0, rx, ry, rz);
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     lhx[j] = rx[j] ? lhx[j] + dhx[j] : T(0);
     lhy[j] = ry[j] ? lhy[j] + dhy[j] : T(0);
     lhz[j] = rz[j] ? lhz[j] + dhz[j] : T(0);
   }
-  st4(a.lhx + i, lhx);
-  st4(a.lhy + i, lhy);
-  st4(a.lhz + i, lhz);
+  st_adj(a.lhx + i, lhx);
+  st_adj(a.lhy + i, lhy);
+  st_adj(a.lhz + i, lhz);
 }
 
 // K2 (step n): gradients and the E auxiliaries' adjoint, then
 // lambda_E = Ca lambda_E + (H step)^T lambda_H + the E phasor source of
 // step n - 1 (t_prev < 0: none).
 template <class T>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 1) k_adj_k2(const __grid_constant__ State<T> s, Adj<T> a,
-                                                int t_prev) {
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : 6)
+    k_adj_k2(const __grid_constant__ State<T> s, Adj<T> a, int t_prev) {
   int z, y, x0;
   if (!vec_cell(s, z, y, x0)) return;
   const int m = s.npml;
   const long long i = idx(s, z, y, x0);
-  T ex[kVec], ey[kVec], ez[kVec], dex[kVec], dey[kVec], dez[kVec];
-  if (z >= m && z < s.nz - m && y >= m && y < s.ny - m && x0 >= m && x0 + kVec - 1 < s.nx - m) {
+  T ex[kAdj], ey[kAdj], ez[kAdj], dex[kAdj], dey[kAdj], dez[kAdj];
+  const int xg = x0 & ~3;
+  if (z >= m && z < s.nz - m && y >= m && y < s.ny - m && xg >= m && xg + 3 < s.nx - m) {
     // no E or H face at the vector, no H face or domain edge at its -x, -y,
-    // -z neighbours
+    // -z neighbours; by four cells, as in k_adj_k1
     e_own_vec<T, true>(s, a, z, y, x0, ex, ey, ez);
     h_to_e_vec<T, true>(s, a, z, y, x0, dex, dey, dez);
   } else {
@@ -807,32 +869,32 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 1) k_adj_k2(const __
   }
   if (t_prev >= 0 && z == s.nz - m - 1) {
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
+    for (int j = 0; j < kAdj; ++j) {
       T pex, pey;
       phasor_e_src(s, a, t_prev, z, y, x0 + j, pex, pey);
       dex[j] += pex;
       dey[j] += pey;
     }
   }
-  bool rx[kVec], ry[kVec], rz[kVec];
+  bool rx[kAdj], ry[kAdj], rz[kAdj];
   e_ranges(s, z, y, x0, rx, ry, rz);
 #pragma unroll
-  for (int j = 0; j < kVec; ++j) {
+  for (int j = 0; j < kAdj; ++j) {
     ex[j] = rx[j] ? ex[j] + dex[j] : T(0);
     ey[j] = ry[j] ? ey[j] + dey[j] : T(0);
     ez[j] = rz[j] ? ez[j] + dez[j] : T(0);
   }
-  st4(a.lex + i, ex);
-  st4(a.ley + i, ey);
-  st4(a.lez + i, ez);
+  st_adj(a.lex + i, ex);
+  st_adj(a.ley + i, ey);
+  st_adj(a.lez + i, ez);
 }
 
-// lanes per row: the width (8, 16 or 32 threads of four cells) that pads the
+// lanes per row: the width (8, 16 or 32 threads of kAdj cells) that pads the
 // row least, the wider on a tie
 inline int adj_lanes(int nx) {
   int best = 32, pad = 1 << 30;
   for (int w : {32, 16, 8}) {
-    const int cells = kVec * w, p = ((nx + cells - 1) / cells) * cells - nx;
+    const int cells = kAdj * w, p = ((nx + cells - 1) / cells) * cells - nx;
     if (p < pad) {
       pad = p;
       best = w;
@@ -850,7 +912,7 @@ void launch_adjoint_first(const State<T>& s, const Adj<T>& a, int t, cudaStream_
 template <class T>
 void launch_adjoint_step(const State<T>& s, const Adj<T>& a, int t, bool first, cudaStream_t st) {
   const int w = adj_lanes(s.nx), rows = 128 / w;
-  const dim3 grd((s.nx + kVec * w - 1) / (kVec * w), (s.ny + rows - 1) / rows, s.nz), blk(w, rows, 1);
+  const dim3 grd((s.nx + kAdj * w - 1) / (kAdj * w), (s.ny + rows - 1) / rows, s.nz), blk(w, rows, 1);
   k_adj_k1<T><<<grd, blk, 0, st>>>(s, a, t, first ? 1 : 0);
   k_adj_k2<T><<<grd, blk, 0, st>>>(s, a, t - 1);
 }
