@@ -261,8 +261,21 @@ def job_rate(units, steps, ms, world):
     return world * units * steps / (ms / 1e3) / 1e6
 
 
+def run_launches(choice, steps):
+    """Kernel launches of one run of `steps` steps: resident steps, one launch
+    and the counter's; a pair of steps, one march of each of the four regions
+    and the phasors; otherwise step_launches a step, and the counter's."""
+    from fdtdsarsim_b200 import _native
+    multi = choice.get('multi', _native.MULTI_OFF) if choice['kernel'] == _native.FDTD_KERNEL_FUSED else 0
+    if multi == _native.MULTI_RESIDENT:
+        return 2
+    if multi == _native.MULTI_PAIR:
+        return 5 * (steps // 2) + step_launches(choice) * (steps % 2) + 1
+    return step_launches(choice) * steps + 1
+
+
 def step_launches(choice):
-    """Kernel launches of one step: split H pass, E pass, phasors; fused
+    """Kernel launches of one single step: split H pass, E pass, phasors; fused
     with the marched shell: interior march, shell march, phasors; fused with
     the split-pass shell: interior march (and z-slab march), shell H pass,
     shell E pass, phasors."""
@@ -272,6 +285,12 @@ def step_launches(choice):
     if choice.get('shell', _native.SHELL_SPLIT) == _native.SHELL_MARCH:
         return 3
     return 4 + int(bool(choice.get('slab', 0)))
+
+
+def multi_name(choice):
+    from fdtdsarsim_b200 import _native
+    return {_native.MULTI_RESIDENT: 'resident', _native.MULTI_PAIR: 'pair',
+            _native.MULTI_AUTO: 'auto'}.get(choice.get('multi', 0), 'off')
 
 
 def shell_name(choice):
@@ -344,8 +363,7 @@ def run_ours(a):
     ms = t_start.elapsed_time(t_end)
     ms_max = max_over_ranks(ms, world, 'cuda')
     value = job_rate(cells, a.steps, ms_max, world)
-    launches_per_step = step_launches(choice)
-    gpu_launches = launches_per_step * a.steps + 1
+    gpu_launches = run_launches(choice, a.steps)
 
     # live per-kernel timing for the roofline (separate pass, same state)
     sim.reset()
@@ -358,8 +376,11 @@ def run_ours(a):
     step_ms, step_n = sim.kernel_time(_native.TIME_STEP)
     ph_ms, ph_n = sim.kernel_time(_native.TIME_PHASOR)
     sim.set_option(_native.OPT_TIMING, 0)
-    kname = 'fused_step' if choice['kernel'] == _native.FDTD_KERNEL_FUSED else 'split_h_e'
-    avg_ms = step_ms / max(step_n, 1)
+    # a launch: one step, or one pass over the fields that makes two
+    per_pass = 2 if multi_name(choice) == 'pair' else 1
+    kname = 'pair_step' if per_pass == 2 else \
+        'fused_step' if choice['kernel'] == _native.FDTD_KERNEL_FUSED else 'split_h_e'
+    avg_ms = per_pass * step_ms / max(step_n, 1)
     alg_bytes = cells * BYTES_PER_CELL[a.dtype]
     peak, peak_kind = measured_peak_hbm()
     achieved = alg_bytes / (avg_ms / 1e3) / 1e9
@@ -367,7 +388,7 @@ def run_ours(a):
                 'frac': round(achieved / peak, 4), 'traffic': committed_traffic(kname, a.workload),
                 'kernel': kname, 'peak_source': peak_kind,
                 'algorithmic_bytes_per_launch': alg_bytes,
-                'avg_launch_ms': round(avg_ms, 4),
+                'avg_launch_ms': round(avg_ms, 4), 'steps_per_launch': per_pass,
                 'phasor_kernel_avg_ms': round(ph_ms / max(ph_n, 1), 4),
                 'step_share_of_device_time': round(step_ms / max(step_ms + ph_ms, 1e-9), 4)}
     sim.close()
@@ -452,11 +473,11 @@ def run_ours(a):
                            kernel=kname, tile=[choice['tile_x'], choice['tile_y']]
                            if choice['kernel'] == _native.FDTD_KERNEL_FUSED else None,
                            zchunk=choice.get('zchunk', 0), z_slabs_fused=int(choice.get('slab', 0)),
-                           shell=shell_name(choice),
+                           shell=shell_name(choice), steps_per_pass=multi_name(choice),
                            autotuned=None if tuned is None else
                            [{'ms': t, 'kernel': 'fused' if c['kernel'] else 'split',
                              'tile_y': c['tile_y'], 'zchunk': c['zchunk'], 'slab': c.get('slab', 0),
-                             'shell': shell_name(c)}
+                             'shell': shell_name(c), 'steps_per_pass': multi_name(c)}
                             for t, c in tuned]),
             'roofline': roofline, 'cpu_baseline': base, 'e2e': e2e,
             'gpu_launches': gpu_launches, 'clocks': clk,
@@ -548,7 +569,9 @@ def batch_record(a, n_models, steps, warmup, check_members=(0, 21, 42)):
         sim = _native.NativeSim(geom, 0)
         sim.set_absorbers(packed_profiles(pc))
         choice = tuning.choose(geom)
-        choices.append(choice)
+        # side by side, the default's choice is between pairs and single steps
+        pairs = choice.get('multi') == _native.MULTI_AUTO and tuning.pair_pays(geom)
+        choices.append(dict(choice, multi=_native.MULTI_PAIR if pairs else choice.get('multi', 0)))
         tuning.apply(sim, choice)
         sim.set_materials(ca, cb)
         sim.set_incident(inc['ex'], inc['ey'], inc['hx'], inc['hy'])
@@ -648,7 +671,7 @@ def batch_record(a, n_models, steps, warmup, check_members=(0, 21, 42)):
                      'kernel': {'streams': 'fused_step (member streams)', 'split': 'batch_split_step',
                                 'queue': 'batch_queue'}[mode]},
         'cpu_baseline': None, 'e2e': None,
-        'gpu_launches': {'streams': sum(step_launches(c) for c in choices) * steps,
+        'gpu_launches': {'streams': sum(run_launches(c, steps) for c in choices),
                          'split': 3 * steps + 1,
                          'queue': 2 * steps + 1}[mode],
         'clocks': clk,

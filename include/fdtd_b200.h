@@ -87,10 +87,12 @@ extern "C" {
 /* several steps per launch (fdtd_set_option(FDTD_OPT_MULTISTEP, ...)) */
 #define FDTD_MULTI_OFF      0
 #define FDTD_MULTI_AUTO     1 /* by the grid's size: resident, pair or single */
-#define FDTD_MULTI_RESIDENT 2 /* every step of fdtd_run in one cooperative launch */
+#define FDTD_MULTI_RESIDENT 2 /* every step of fdtd_run in one cooperative
+                                 launch (not among a batch's streams) */
 #define FDTD_MULTI_PAIR     3 /* two steps per pass over the fields; holds a
-                                 third field set (single steps where there is
-                                 no memory for it, or the grid is too narrow) */
+                                 few planes more (single steps where there is
+                                 no memory for them, or the grid is too
+                                 narrow) */
 
 /* batched sweep (fdtd_batch_set_option(FDTD_OPT_BATCH_MODE, ...)) */
 #define FDTD_BATCH_SPLIT   0   /* (default) one launch per pass (H, E, phasors)

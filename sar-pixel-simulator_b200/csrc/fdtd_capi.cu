@@ -460,11 +460,11 @@ constexpr int kPairNxFloat = 160;
 template <class T>
 bool takes_resident(const fdtd_sim* s, int n) {
   if (s->kernel != FDTD_KERNEL_FUSED || s->check_every > 0 || n < 2) return false;
-  if (s->multi == FDTD_MULTI_RESIDENT) return true;
   // members that run side by side: a launch that takes every SM would run
   // them one after another (10 members of 0.6 to 4 M cells: 507 us per step
   // against 452)
   if (s->side_by_side) return false;
+  if (s->multi == FDTD_MULTI_RESIDENT) return true;
   return s->multi == FDTD_MULTI_AUTO && s->vol * 11 * (long long)sizeof(T) <= kResidentBytes;
 }
 

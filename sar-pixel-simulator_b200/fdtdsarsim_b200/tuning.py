@@ -20,10 +20,12 @@ DEFAULT_TILE = (32, 4)
 
 _MARCH, _SPLIT = _native.SHELL_MARCH, _native.SHELL_SPLIT
 
-# (kernel, tile_y, zchunk, slab, shell); zchunk 0 lets the library pick;
+# (kernel, tile_y, zchunk, slab, shell[, multi]); zchunk 0 lets the library pick;
 # shell: the fused step's shell marched (_MARCH) or swept by the split
 # passes (_SPLIT), then slab 1 marches the CPML z slabs, slab 2 the whole
-# z extent of the interior's x-y box (the column march)
+# z extent of the interior's x-y box (the column march); multi: several steps
+# per pass (off where not given), with single steps of the same candidate for
+# what is left over
 CANDIDATES = [
     (_native.FDTD_KERNEL_SPLIT, 4, 0, 0, _MARCH),
     (_native.FDTD_KERNEL_FUSED, 4, 0, 0, _MARCH),
@@ -33,10 +35,12 @@ CANDIDATES = [
     (_native.FDTD_KERNEL_FUSED, 8, 0, 0, _SPLIT),
     (_native.FDTD_KERNEL_FUSED, 4, 0, 1, _SPLIT),
     (_native.FDTD_KERNEL_FUSED, 4, 0, 2, _SPLIT),
+    (_native.FDTD_KERNEL_FUSED, 4, 0, 0, _SPLIT, _native.MULTI_RESIDENT),
+    (_native.FDTD_KERNEL_FUSED, 4, 0, 0, _SPLIT, _native.MULTI_PAIR),
 ]
 
 # cache entries measured with another candidate set are measured again
-_VERSION = 'v3'
+_VERSION = 'v4'
 
 
 def cache_path():
@@ -74,13 +78,23 @@ def choose(geom, kernel=None, tile=None, device=0, use_cache=True):
     if kernel is None and tile is None and use_cache:
         hit = lookup(geom, device)
         if hit:
-            return {'kernel': int(hit['kernel']), 'tile_x': 32, 'tile_y': int(hit['tile_y']),
-                    'zchunk': int(hit['zchunk']), 'slab': int(hit.get('slab', 0)),
-                    'shell': int(hit.get('shell', _SPLIT))}
+            choice = {'kernel': int(hit['kernel']), 'tile_x': 32, 'tile_y': int(hit['tile_y']),
+                      'zchunk': int(hit['zchunk']), 'slab': int(hit.get('slab', 0)),
+                      'shell': int(hit.get('shell', _SPLIT))}
+            if 'multi' in hit:
+                choice['multi'] = int(hit['multi'])
+            return choice
     k = _native.FDTD_KERNEL_FUSED if kernel is None else int(kernel)
     tx, ty = tile if tile is not None else DEFAULT_TILE
     return {'kernel': k, 'tile_x': int(tx), 'tile_y': int(ty), 'zchunk': 0, 'slab': 0, 'shell': _SPLIT,
             'multi': _native.MULTI_AUTO if kernel is None and tile is None else _native.MULTI_OFF}
+
+
+def pair_pays(geom):
+    """Whether MULTI_AUTO takes two steps per pass on this grid (where it does
+    not run them resident): the library's rule on cells and width."""
+    cells = geom.nx * geom.ny * geom.nz
+    return cells >= 1.5e6 if geom.dtype == _native.FDTD_F64 else cells >= 4e6 and geom.nx >= 160
 
 
 def apply(sim, choice):
@@ -120,7 +134,7 @@ def autotune(geom, device=0, steps=6, candidates=None, save=True):
         kernel, ty, zc, slab = cand[:4]
         shell = cand[4] if len(cand) > 4 else _MARCH
         choice = {'kernel': kernel, 'tile_x': 32, 'tile_y': ty, 'zchunk': zc, 'slab': slab,
-                  'shell': shell}
+                  'shell': shell, 'multi': cand[5] if len(cand) > 5 else _native.MULTI_OFF}
         try:
             apply(sim, choice)
             sim.reset()
