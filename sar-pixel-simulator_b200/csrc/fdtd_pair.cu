@@ -31,6 +31,8 @@
 //   x ends  the columns at either x end, all y, all z: every face. Tiles of
 //           128-byte rows by 32 rows: the rows of an x face are short, and a
 //           wide tile would march mostly plain cells with the general update.
+//           (At the low end 64-byte rows by 64 would do; that tile, a launch
+//           of its own, made the step slower: 198 us against 184 there.)
 //           (Tiles turned so that a warp is one column of vectors, where an x
 //           face is uniform over a warp, ran fewer instructions, but the face
 //           warps kept the others waiting at the barriers: 183 us against
@@ -258,7 +260,10 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
 #pragma unroll
   for (int q = 0; q < 6; ++q) { vset(A.ph[q], T(0)); vset(A.pe[q], T(0)); }
   B = A;
-  bool good = mbar_wait(bars, 0);   // E(zs)
+  // the plane at which a copy did not arrive within the time limit (kNever:
+  // all did). From there on nothing is waited for and no more copies start.
+  constexpr int kNever = 0x7fffffff;
+  int lost = mbar_wait(bars, 0) ? kNever : zs;   // E(zs)
   int es = 0;                       // E ring slot of plane z
   unsigned ep = 1;                  // bit k: parity of E slot k's next wait
 
@@ -279,10 +284,10 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     }
     if (first) {
       if (z + 1 <= ze) {
-        good = good && mbar_wait(bars + 8 * en, (ep >> en) & 1u);
+        if (lost == kNever && !mbar_wait(bars + 8 * en, (ep >> en) & 1u)) lost = z;
         ep ^= 1u << en;
       }
-      good = good && mbar_wait(bars + 24 + 8 * (k & 1), (k >> 1) & 1);
+      if (lost == kNever && !mbar_wait(bars + 24 + 8 * (k & 1), (k >> 1) & 1)) lost = z;
       const T* const E0 = reinterpret_cast<const T*>(smem + es * C::kEBytes) + at;
       const T* const E1 = reinterpret_cast<const T*>(smem + en * C::kEBytes) + at;
       const T* const HC = reinterpret_cast<const T*>(smem + C::kHRing + (k & 1) * C::kHBytes) + at;
@@ -309,7 +314,7 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     }
     __syncthreads();
     // every thread has read plane z of the rings: their slots take new planes
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && lost == kNever) {
       if (z + 3 <= ze) issue_e(z + 3);
       if (z + 2 <= zl) issue_hc(z + 2);
     }
@@ -384,7 +389,15 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     plane(z, A, B);
     if (z < z1) plane(z + 1, B, A);
   }
-  if (!good) *err = 1;   // a copy did not arrive within the time limit
+  if (lost != kNever) {
+    *err = 1;
+    // the copies in flight still land in this block's memory: a bounded wait
+    // for the last that were started
+    if (threadIdx.x == 0) {
+      for (int z = lost; z <= min(lost + 2, ze); ++z) mbar_wait(bars + 8 * ((z - zs) % 3), ((z - zs) / 3) & 1);
+      for (int z = lost; z <= min(lost + 1, zl); ++z) mbar_wait(bars + 24 + 8 * ((z - zs) & 1), ((z - zs) >> 1) & 1);
+    }
+  }
 }
 
 // The four tile kinds (registers per thread are bounded by 65536 / threads).
