@@ -451,7 +451,8 @@ int fdtd_incident_create(const fdtd_geometry *geom, int nt_pulse, int device,
 int fdtd_incident_destroy(fdtd_incident *inc);
 /* FDTD_OPT_KERNEL (default FDTD_KERNEL_FUSED: the fused step, its source
  * plane written after each step), FDTD_OPT_TILE_Y, FDTD_OPT_ZCHUNK,
- * FDTD_OPT_FUSED_SLAB. */
+ * FDTD_OPT_FUSED_SLAB, FDTD_OPT_MULTISTEP (here default FDTD_MULTI_AUTO:
+ * grids that stay in L2 run all steps in one launch; no pairs). */
 int fdtd_incident_set_option(fdtd_incident *inc, int option, int value);
 /* 8 * npml profiles, packed as for fdtd_set_absorbers (Absorbers(params)
  * of the incident simulation, cpu/fdtd_sim.py:14-23). */

@@ -2229,7 +2229,7 @@ int incident_run(fdtd_incident* b) {
   add_shell_box(whole, 0, g.nx, 0, g.ny, 0, g.nz);
   const State<T> st = make_state<T>(s, 0, 0);   // split passes in place on set 0
   const int* zero_t = s->tdev + 2;
-  IncidentRecord<T> r;
+  IncidentRecord<T> r = {};
   r.rex = (T*)b->rec[0]; r.rey = (T*)b->rec[1]; r.rhx = (T*)b->rec[2]; r.rhy = (T*)b->rec[3];
   r.ph = (T*)b->iph;
   r.phase = s->phase;
@@ -2244,7 +2244,18 @@ int incident_run(fdtd_incident* b) {
   // (cpu/incident_sim.py:134-160)
   launch_shell_pass<T>(st, zero_t, 0, whole, false, s->stream);
   source(0, 0);
-  if (s->kernel == FDTD_KERNEL_FUSED) {
+  bool done = false;
+  if (takes_resident<T>(s, g.nt)) {
+    // every step in one resident launch, the source and the read-out with
+    // them
+    const IncidentBeam<T> beam = {r, (const T*)b->exc[0], (const T*)b->exc[1], b->feed_in, b->nt_pulse};
+    T* const other[3] = {(T*)s->fld[1][3], (T*)s->fld[1][4], (T*)s->fld[1][5]};
+    done = launch_resident_beam<T>(st, other, beam, s->tdev, g.nt, (unsigned*)(s->tdev + 4), s->tdev + 6, s->stream);
+    if (done) s->wait_look = true;
+    else cudaGetLastError();   // a device without cooperative launches: single steps
+  }
+  if (done) {
+  } else if (s->kernel == FDTD_KERNEL_FUSED) {
     // the fused step of t gives H^{t+1/2} and the next step's E update; the
     // read-out takes E^t from the source set and H^{t+1/2} from the
     // destination set, and the next step's source goes onto the destination
@@ -2269,6 +2280,7 @@ int incident_run(fdtd_incident* b) {
   }
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(s->stream));
+  if ((rc = take_wait_error(s))) return rc;
   s->t = g.nt;
   b->ran = true;
   return FDTD_OK;
@@ -2297,6 +2309,7 @@ int fdtd_incident_create(const fdtd_geometry* geom, int nt_pulse, int device, fd
   // plane of the grid
   s->g.tfsf_z = -2;
   s->kernel = FDTD_KERNEL_FUSED;
+  s->multi = FDTD_MULTI_AUTO;
   s->tile_x = 32;
   s->tile_y = 4;
   b->nt_pulse = std::min(nt_pulse, g.nt);   // the reference's loop ends at nt
@@ -2379,7 +2392,7 @@ int fdtd_incident_set_option(fdtd_incident* b, int option, int value) {
   int rc = check_inc(b);
   if (rc) return rc;
   if (option != FDTD_OPT_KERNEL && option != FDTD_OPT_TILE_Y && option != FDTD_OPT_ZCHUNK &&
-      option != FDTD_OPT_FUSED_SLAB)
+      option != FDTD_OPT_FUSED_SLAB && option != FDTD_OPT_MULTISTEP)
     return fail(FDTD_ERR_INVALID, "option %d does not apply to an incident run", option);
   return fdtd_set_option(b->sim, option, value);
 }

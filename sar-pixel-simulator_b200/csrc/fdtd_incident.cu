@@ -20,7 +20,8 @@
 // Incident run (cpu/incident_sim.py:67-171): the E pass, the hard source on
 // plane feed_in, the H pass (the split passes of the main step, without
 // injection), then k_inc_record copies the read-out plane and accumulates the
-// incident phasors (cpu/field_updates.py:465-491).
+// incident phasors (cpu/field_updates.py:465-491). Grids that stay in L2 do
+// all of it in one launch (fdtd_resident.cu).
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -28,6 +29,7 @@
 #include <cufft.h>
 
 #include "fdtd_b200.h"
+#include "fdtd_incident.cuh"
 #include "fdtd_launch.h"
 
 namespace fdtd {
@@ -165,39 +167,11 @@ __global__ void __launch_bounds__(256) k_inc_source(T* __restrict__ ex, T* __res
 }
 
 template <class T>
-__device__ __forceinline__ void inc_acc(T* p, double m, double c, double sn) {
-  // float64 sum of the stored value and the float64 term, rounded to T
-  p[0] = R<T>::from_double(__dadd_rn((double)p[0], __dmul_rn(m, c)));
-  p[1] = R<T>::from_double(__dadd_rn((double)p[1], __dmul_rn(m, sn)));
-}
-
-// Read-out plane of step t into the recorded planes (all y, x) and the
-// incident phasors of cpu/field_updates.py:465-491 at (y, x) in
-// [1, ny_ph) x [1, nx_ph): E averaged with phase exp(-i omega (t - 1/2) dt),
-// H with exp(-i omega t dt) (phase table columns 2-3 and 0-1).
-template <class T>
 __global__ void __launch_bounds__(256) k_inc_record(IncidentRecord<T> r, int t) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   if (x >= r.nx) return;
-  const long long P = r.plane, W = r.pitch;
-  const long long i = (long long)r.read_out * P + (long long)y * W + x;
-  const long long o = ((long long)t * r.ny + y) * W + x;
-  r.rex[o] = r.ex[i];
-  r.rey[o] = r.ey[i];
-  r.rhx[o] = r.hx[i];
-  r.rhy[o] = r.hy[i];
-  const int a = y - r.npml, b = x - r.npml;
-  if (a < 1 || b < 1 || a >= r.ny_ph || b >= r.nx_ph) return;
-  const double* ph = r.phase + 4 * (long long)t;
-  const double cH = ph[0], sH = ph[1], cE = ph[2], sE = ph[3];
-  using M = R<T>;
-  const long long k = 2 * ((long long)a * r.nx_ph + b), n = 2 * (long long)r.ny_ph * r.nx_ph;
-  inc_acc(r.ph + k, 0.5 * (double)M::add(r.ex[i], r.ex[i - 1]), cE, sE);
-  inc_acc(r.ph + n + k, 0.5 * (double)M::add(r.ey[i], r.ey[i - W]), cE, sE);
-  inc_acc(r.ph + 2 * n + k,
-          0.25 * (double)M::add(M::add(M::add(r.hx[i], r.hx[i - W]), r.hx[i - P]), r.hx[i - P - W]), cH, sH);
-  inc_acc(r.ph + 3 * n + k,
-          0.25 * (double)M::add(M::add(M::add(r.hy[i], r.hy[i - 1]), r.hy[i - P]), r.hy[i - P - 1]), cH, sH);
+  inc_record_e(r, r.ex, r.ey, t, y, x);
+  inc_record_h(r, r.hx, r.hy, t, y, x);
 }
 
 template <class T>

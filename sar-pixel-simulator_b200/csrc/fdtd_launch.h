@@ -157,6 +157,30 @@ template <class T>
 void launch_shell_pass(const State<T>& s, const int* tdev, int toff, const ShellBoxes& bl,
                        bool h_pass, cudaStream_t st);
 
+// The read-out plane of the incident run and the incident phasors: fields
+// of the run (its current set), the recorded planes (nt, ny, pitch), the
+// four phasor planes (complex, (ny_ph, nx_ph) each, consecutive) and the
+// run's phase table (per step: cos/sin of the t and t - 1/2 angles).
+template <class T>
+struct IncidentRecord {
+  const T* ex; const T* ey; const T* hx; const T* hy;
+  T* rex; T* rey; T* rhx; T* rhy;
+  T* ph;
+  const double* phase;
+  int nx, ny, pitch;
+  long long plane;
+  int npml, read_out, nx_ph, ny_ph;
+};
+
+// The incident run's part of its steps: the read-out (its field pointers are
+// the run's own), the source planes (nt_source, ny, pitch) on plane feed_in.
+template <class T>
+struct IncidentBeam {
+  IncidentRecord<T> rec;
+  const T* ex; const T* ey;
+  int feed_in, nt_source;
+};
+
 // Resident step (fdtd_resident.cu): many split steps of a small grid in one
 // cooperative launch.
 struct DivMagic {
@@ -171,6 +195,7 @@ struct ResidentArgs {
   int ph_units;      // 32-cell units of the largest phasor plane
   DivMagic per_row, per_plane;   // division by gx and by gy
   float minus0;      // -0 (fdtd_vecn.cuh: vmul)
+  IncidentBeam<T> beam;   // an incident run's
 };
 // Enqueues nsteps steps from the step *tdev + toff (their phasors in plane
 // groups ph_g0 .. ph_g0 + ph_ng - 1 included); the run ends on the set it
@@ -179,6 +204,12 @@ struct ResidentArgs {
 template <class T>
 bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, int toff, int nsteps, int ph_g0,
                      int ph_ng, unsigned* sync, int* err, cudaStream_t st);
+// The same for an incident run's steps 0 .. nsteps - 1, whose first E update
+// and source are done: each H update, then the next step's E update with its
+// source; the read-out plane of every step beside them.
+template <class T>
+bool launch_resident_beam(const State<T>& s, T* const other_h[3], const IncidentBeam<T>& beam, const int* tdev,
+                          int nsteps, unsigned* sync, int* err, cudaStream_t st);
 
 // Pair step (fdtd_pair.cu): two steps per pass, by marches over regions of
 // four kinds. A region is the box x [x0, x1), y [y0, y1), z [z0, z1), cut
@@ -282,21 +313,6 @@ struct IncidentTaper {
 template <class T>
 int make_incident_excitation(const IncidentTaper& p, const double* k_host, const double* pfft_host,
                              int nt_pulse, int pitch, T* ex, T* ey, double* peak_out, cudaStream_t st);
-
-// The read-out plane of the incident run and the incident phasors: fields
-// of the run (its current set), the recorded planes (nt, ny, pitch), the
-// four phasor planes (complex, (ny_ph, nx_ph) each, consecutive) and the
-// run's phase table (per step: cos/sin of the t and t - 1/2 angles).
-template <class T>
-struct IncidentRecord {
-  const T* ex; const T* ey; const T* hx; const T* hy;
-  T* rex; T* rey; T* rhx; T* rhy;
-  T* ph;
-  const double* phase;
-  int nx, ny, pitch;
-  long long plane;
-  int npml, read_out, nx_ph, ny_ph;
-};
 
 template <class T>
 void launch_inc_source(T* ex, T* ey, const T* sx, const T* sy, int nx, int ny, int pitch, long long plane,

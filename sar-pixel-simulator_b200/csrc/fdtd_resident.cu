@@ -20,9 +20,12 @@
 // 47 x 87 x 107 62 and 27. A phase is latency: at the smallest size about
 // 2 us of barrier and 2 us of one vector's loads and update; at 55 x 133 x 133
 // five rounds of them per block (IPC 1.1).
+// An incident run of 100 x 133 x 133 cells, its source and read-out included:
+// 67 and 49.
 #include <algorithm>
 #include <cstring>
 
+#include "fdtd_incident.cuh"
 #include "fdtd_launch.h"
 #include "fdtd_split.cuh"
 #include "fdtd_vecn.cuh"
@@ -95,7 +98,10 @@ template <int V> constexpr int kResRows = 32 / kResWidth<V>;
 // One launch: `nsteps` steps from *tp + toff; a.st has H in place in the
 // current set, a.other the other set's H. A block takes a contiguous run of
 // units in (z, y, x) order (neighbouring rows then meet in its L1).
-template <class T, int V>
+// kBeam: an incident run's steps (a.beam): E of the read-out plane is recorded
+// beside the H pass and H beside the E pass, where neither changes, and the
+// E pass puts the next step's source on its plane.
+template <class T, int V, bool kBeam>
 __global__ void __launch_bounds__(kResThreads<T, V>, 1)
 k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp, int toff, int nsteps, int ph_g0,
            int ph_ng, unsigned* sync, int* err) {
@@ -114,6 +120,14 @@ k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp
     for (int u = warp * gridDim.x + blockIdx.x; u < ph_units; u += warps * gridDim.x) {
       const int g = u / a.ph_units;
       phasor_cell(s, PhFields<T>{s.iex, s.iey, s.iez, h[0], h[1], h[2]}, ph_g0 + g, (u - g * a.ph_units) * 32 + lane, t);
+    }
+  };
+  // f(y, x) for the read-out plane's cells
+  auto read_out = [&](auto&& f) {
+    const int per_row = (s.nx + 31) / 32;
+    for (int u = warp * gridDim.x + blockIdx.x; u < ny * per_row; u += warps * gridDim.x) {
+      const int y = u / per_row, x = (u - y * per_row) * 32 + lane;
+      if (x < s.nx) f(y, x);
     }
   };
   // pass(z, p, i, easy) for the block's vectors: i the element index; easy:
@@ -150,6 +164,8 @@ k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp
     T* const hd[3] = {dst_cur ? cur[0] : a.other[0], dst_cur ? cur[1] : a.other[1], dst_cur ? cur[2] : a.other[2]};
     const int t = t0 + n;
     if (n > 0) phasors(hs, t - 1);
+    if constexpr (kBeam)
+      read_out([&](int y, int x) { inc_record_e<T>(a.beam.rec, s.iex, s.iey, t, y, x); });
     if (in_place && n > 0 && !grid_barrier(sync, ++turn)) break;
     sweep([&](int z, const PairPos<T, V>& p, unsigned i, bool easy) {
       T ph[6][V], pe[6][V];
@@ -169,6 +185,8 @@ k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp
       if (!easy) pair_psi<ResAll, 1>(s, p, z, ph, pe, store);
     });
     if (!grid_barrier(sync, ++turn)) break;
+    if constexpr (kBeam)
+      read_out([&](int y, int x) { inc_record_h<T>(a.beam.rec, hd[0], hd[1], t, y, x); });
     sweep([&](int z, const PairPos<T, V>& p, unsigned i, bool easy) {
       T ph[6][V], pe[6][V];
       if (!easy) pair_psi<ResAll, 2>(s, p, z, ph, pe, load);
@@ -182,6 +200,17 @@ k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp
       ldg(ca, s.ca + i); ldg(cb, s.cb + i);
       if (easy) pair_e<ResPlain>(s, p, z, t, hx, hy, hz, hxz, hyz, hxy, hzy, hyp, hzp, ca, cb, ex, ey, ez, pe);
       else pair_e<ResAll>(s, p, z, t, hx, hy, hz, hxz, hyz, hxy, hzy, hyp, hzp, ca, cb, ex, ey, ez, pe);
+      if constexpr (kBeam) {
+        if (z == a.beam.feed_in && t + 1 < a.beam.nt_source) {
+          const long long src = ((long long)(t + 1) * ny + p.y) * s.pitch + p.x0;
+#pragma unroll
+          for (int j = 0; j < V; ++j)
+            if (inc_source_cell(s, p.y, p.x0 + j)) {
+              ex[j] = a.beam.ex[src + j];
+              ey[j] = a.beam.ey[src + j];
+            }
+        }
+      }
       stg(s.oex + i, ex); stg(s.oey + i, ey); stg(s.oez + i, ez);
       if (!easy) pair_psi<ResAll, 2>(s, p, z, ph, pe, store);
     });
@@ -192,13 +221,14 @@ k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp
 }
 
 // Blocks of a launch (one per SM), 0 when the device cannot run it.
-template <class T, int V>
+template <class T, int V, bool kBeam>
 int resident_blocks() {
   int dev = 0, sms = 0, coop = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident<T, V>, kResThreads<T, V>, 0) != cudaSuccess) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident<T, V, kBeam>, kResThreads<T, V>,
+                                                    0) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -218,10 +248,10 @@ DivMagic div_magic(unsigned d) {
   return r;
 }
 
-template <class T, int V>
+template <class T, int V, bool kBeam>
 bool resident_launch(ResidentArgs<T>& a, const int* tdev, int toff, int nsteps, int ph_g0, int ph_ng, unsigned* sync,
                      int* err, cudaStream_t st) {
-  const int blocks = resident_blocks<T, V>();
+  const int blocks = resident_blocks<T, V, kBeam>();
   if (!blocks) return false;
   const State<T>& s = a.st;
   a.gx = (s.nx + kResCells - 1) / kResCells;
@@ -231,17 +261,17 @@ bool resident_launch(ResidentArgs<T>& a, const int* tdev, int toff, int nsteps, 
   a.per_plane = div_magic((unsigned)a.gy);
   void* args[] = {&a, &tdev, &toff, &nsteps, &ph_g0, &ph_ng, &sync, &err};
   return cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), st) == cudaSuccess &&
-         cudaLaunchCooperativeKernel((const void*)k_resident<T, V>, dim3(blocks), dim3(kResThreads<T, V>), args, 0, st) ==
-             cudaSuccess;
+         cudaLaunchCooperativeKernel((const void*)k_resident<T, V, kBeam>, dim3(blocks), dim3(kResThreads<T, V>), args, 0,
+                                     st) == cudaSuccess;
 }
 
 }  // namespace
 
-template <class T>
-bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, int toff, int nsteps, int ph_g0,
-                     int ph_ng, unsigned* sync, int* err, cudaStream_t st) {
-  ResidentArgs<T> a;
-  memset(&a, 0, sizeof(a));
+namespace {
+
+template <class T, bool kBeam>
+bool resident(ResidentArgs<T>& a, const State<T>& s, T* const other_h[3], const int* tdev, int toff, int nsteps,
+              int ph_g0, int ph_ng, unsigned* sync, int* err, cudaStream_t st) {
   a.st = s;
   for (int k = 0; k < 3; ++k) a.other[k] = other_h[k];
   a.minus0 = -0.0f;
@@ -251,10 +281,34 @@ bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, in
   // one short chain (31 x 39 x 39: 8.8 us per step, 13.0 with four; 47 x 87 x 107 in
   // double: 29 with one cell, 27 with two).
   const long long cells = (long long)s.nz * s.ny * s.nx;
-  if (cells <= kResOneCell) return resident_launch<T, 1>(a, tdev, toff, nsteps, ph_g0, ph_ng, sync, err, st);
-  return resident_launch<T, 16 / (int)sizeof(T)>(a, tdev, toff, nsteps, ph_g0, ph_ng, sync, err, st);
+  if (cells <= kResOneCell)
+    return resident_launch<T, 1, kBeam>(a, tdev, toff, nsteps, ph_g0, ph_ng, sync, err, st);
+  return resident_launch<T, 16 / (int)sizeof(T), kBeam>(a, tdev, toff, nsteps, ph_g0, ph_ng, sync, err, st);
 }
 
+}  // namespace
+
+template <class T>
+bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, int toff, int nsteps, int ph_g0,
+                     int ph_ng, unsigned* sync, int* err, cudaStream_t st) {
+  ResidentArgs<T> a;
+  memset(&a, 0, sizeof(a));
+  return resident<T, false>(a, s, other_h, tdev, toff, nsteps, ph_g0, ph_ng, sync, err, st);
+}
+
+template <class T>
+bool launch_resident_beam(const State<T>& s, T* const other_h[3], const IncidentBeam<T>& beam, const int* tdev,
+                          int nsteps, unsigned* sync, int* err, cudaStream_t st) {
+  ResidentArgs<T> a;
+  memset(&a, 0, sizeof(a));
+  a.beam = beam;
+  return resident<T, true>(a, s, other_h, tdev, 0, nsteps, 0, 0, sync, err, st);
+}
+
+template bool launch_resident_beam<float>(const State<float>&, float* const[3], const IncidentBeam<float>&, const int*,
+                                          int, unsigned*, int*, cudaStream_t);
+template bool launch_resident_beam<double>(const State<double>&, double* const[3], const IncidentBeam<double>&,
+                                           const int*, int, unsigned*, int*, cudaStream_t);
 template bool launch_resident<float>(const State<float>&, float* const[3], const int*, int, int, int, int, unsigned*,
                                      int*, cudaStream_t);
 template bool launch_resident<double>(const State<double>&, double* const[3], const int*, int, int, int, int,
