@@ -260,10 +260,11 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
 #pragma unroll
   for (int q = 0; q < 6; ++q) { vset(A.ph[q], T(0)); vset(A.pe[q], T(0)); }
   B = A;
-  // the plane at which a copy did not arrive within the time limit (kNever:
-  // all did). From there on nothing is waited for and no more copies start.
-  constexpr int kNever = 0x7fffffff;
-  int lost = mbar_wait(bars, 0) ? kNever : zs;   // E(zs)
+  // good: every copy so far arrived within the time limit. After the first
+  // that did not, at plane `lost` (thread 0), nothing is waited for and no more
+  // start.
+  int lost = zs;
+  bool good = mbar_wait(bars, 0);   // E(zs)
   int es = 0;                       // E ring slot of plane z
   unsigned ep = 1;                  // bit k: parity of E slot k's next wait
 
@@ -284,10 +285,10 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     }
     if (first) {
       if (z + 1 <= ze) {
-        if (lost == kNever && !mbar_wait(bars + 8 * en, (ep >> en) & 1u)) lost = z;
+        good = good && mbar_wait(bars + 8 * en, (ep >> en) & 1u);
         ep ^= 1u << en;
       }
-      if (lost == kNever && !mbar_wait(bars + 24 + 8 * (k & 1), (k >> 1) & 1)) lost = z;
+      good = good && mbar_wait(bars + 24 + 8 * (k & 1), (k >> 1) & 1);
       const T* const E0 = reinterpret_cast<const T*>(smem + es * C::kEBytes) + at;
       const T* const E1 = reinterpret_cast<const T*>(smem + en * C::kEBytes) + at;
       const T* const HC = reinterpret_cast<const T*>(smem + C::kHRing + (k & 1) * C::kHBytes) + at;
@@ -314,7 +315,8 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     }
     __syncthreads();
     // every thread has read plane z of the rings: their slots take new planes
-    if (threadIdx.x == 0 && lost == kNever) {
+    if (threadIdx.x == 0 && good) {
+      lost = z + 1;
       if (z + 3 <= ze) issue_e(z + 3);
       if (z + 2 <= zl) issue_hc(z + 2);
     }
@@ -389,7 +391,7 @@ k_pair(const __grid_constant__ State<typename C::T> s, const __grid_constant__ P
     plane(z, A, B);
     if (z < z1) plane(z + 1, B, A);
   }
-  if (lost != kNever) {
+  if (!good) {
     *err = 1;
     // the copies in flight still land in this block's memory: a bounded wait
     // for the last that were started
