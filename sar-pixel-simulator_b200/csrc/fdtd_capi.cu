@@ -76,8 +76,11 @@ struct fdtd_sim {
   long long ph_off[24];
   long long ph_elems = 0;
   double* phase = nullptr;
-  int* tdev = nullptr;                   // step counter; [2] stays 0; [4], [5] the resident step's barrier;
-                                         // [6] set by a kernel when a wait inside it ran out
+  int* tdev = nullptr;                   // step counter; [2] stays 0; [4], [5] the resident step's barrier
+  // page-locked host word that a kernel sets when a wait inside it ran out:
+  // read after a synchronisation without a copy on the legacy default
+  // stream, which would wait for other streams
+  int* waited = nullptr;
   int* flags = nullptr;                  // non-finite check: found, step
   int64_t t = 0;
   int cur = 0;
@@ -134,7 +137,6 @@ struct fdtd_sim {
   void* pair_mid = nullptr;              // the planes of a PairMid
   cudaStream_t side2 = nullptr;
   cudaEvent_t join2 = nullptr;
-  bool wait_look = false;                // such kernels were enqueued since the last look
   // captured step chunks (FDTD_OPT_GRAPH_CHUNK), one per starting field set,
   // with the settings they were captured under; absorber uploads bump the
   // epoch (the profiles are captured by value)
@@ -236,12 +238,9 @@ int take_bounds_violation() {
 // A wait inside a kernel that ran out since the last look (the results of
 // that run are not valid). After a synchronisation of the handle's stream.
 int take_wait_error(fdtd_sim* s) {
-  if (!s->wait_look) return FDTD_OK;
-  s->wait_look = false;
-  int w = 0;
-  CK(cudaMemcpy(&w, s->tdev + 6, sizeof(w), cudaMemcpyDeviceToHost));
-  if (!w) return FDTD_OK;
-  CK(cudaMemset(s->tdev + 6, 0, sizeof(w)));
+  volatile int* w = s->waited;
+  if (!*w) return FDTD_OK;
+  *w = 0;
   return fail(FDTD_ERR_CUDA, "a wait inside a step kernel ran out: the run's results are not valid");
 }
 
@@ -424,11 +423,10 @@ int enqueue_pair(fdtd_sim* s, int k, int ph_g0, int ph_ng, cudaEvent_t after_ste
   CK(cudaStreamWaitEvent(s->side, s->fork, 0));
   CK(cudaStreamWaitEvent(s->side2, s->fork, 0));
   const PairMapSet& maps = s->pmaps[s->cur];
-  s->wait_look = true;
-  if (!launch_pair<T>(kPairX, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side) ||
-      !launch_pair<T>(kPairY, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side2) ||
-      !launch_pair<T>(kPairPlain, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->stream) ||
-      !launch_pair<T>(kPairZ, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side2))
+  if (!launch_pair<T>(kPairX, st, s->pair, maps, mid, s->tdev, k, s->waited, s->side) ||
+      !launch_pair<T>(kPairY, st, s->pair, maps, mid, s->tdev, k, s->waited, s->side2) ||
+      !launch_pair<T>(kPairPlain, st, s->pair, maps, mid, s->tdev, k, s->waited, s->stream) ||
+      !launch_pair<T>(kPairZ, st, s->pair, maps, mid, s->tdev, k, s->waited, s->side2))
     return fail(FDTD_ERR_CUDA, "pair step launch: %s", cudaGetErrorString(cudaGetLastError()));
   CK(cudaEventRecord(s->join, s->side));
   CK(cudaEventRecord(s->join2, s->side2));
@@ -486,10 +484,9 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     mark(s, e0);
     T* const other[3] = {(T*)s->fld[1 - s->cur][3], (T*)s->fld[1 - s->cur][4], (T*)s->fld[1 - s->cur][5]};
     const bool ok = launch_resident<T>(make_state<T>(s, s->cur, s->cur), other, s->tdev, 0, n, ph_g0, ph_ng,
-                                       (unsigned*)(s->tdev + 4), s->tdev + 6, s->stream);
+                                       (unsigned*)(s->tdev + 4), s->waited, s->stream);
     mark(s, e1);
     mark(s, e2);
-    s->wait_look = true;
     if (ok) {
       launch_advance(s->tdev, n, s->stream);
       CK(cudaGetLastError());
@@ -621,7 +618,6 @@ int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
     memcpy(s->gsig[start], sig, sizeof(sig));
   }
   CK(cudaGraphLaunch(s->gexec[start], s->stream));
-  s->wait_look = s->wait_look || s->multi != FDTD_MULTI_OFF;
   s->cur = s->gend[start];
   return FDTD_OK;
 }
@@ -781,6 +777,11 @@ int fdtd_create(const fdtd_geometry* geom, int device, fdtd_sim** out) {
   A((size_t)std::max(g.nt, 1) * 4 * sizeof(double), (void**)&s->phase);
   A(sizeof(int) * 8, (void**)&s->tdev);
   A(sizeof(int) * 2, (void**)&s->flags);
+  if (rc == FDTD_OK && cudaHostAlloc((void**)&s->waited, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    s->waited = nullptr;
+    rc = fail(FDTD_ERR_NOMEM, "no page-locked host memory");
+  }
   if (rc != FDTD_OK) {
     fdtd_destroy(s);
     return rc;
@@ -849,6 +850,7 @@ int fdtd_destroy(fdtd_sim* s) {
     if (s->stage[k]) cudaFreeHost(s->stage[k]);
   }
   if (s->copy) cudaStreamDestroy(s->copy);
+  if (s->waited) cudaFreeHost(s->waited);
   for (auto e : s->ev) cudaEventDestroy(e);
   for (int k = 0; k < 2; ++k)
     if (s->gexec[k]) cudaGraphExecDestroy(s->gexec[k]);
@@ -1152,6 +1154,7 @@ int fdtd_reset(fdtd_sim* s) {
   CK(cudaMemsetAsync(s->tdev, 0, sizeof(int) * 8, s->stream));
   CK(cudaMemsetAsync(s->flags, 0, sizeof(int) * 2, s->stream));
   CK(cudaStreamSynchronize(s->stream));
+  *s->waited = 0;
   s->t = 0;
   s->cur = 0;
   return FDTD_OK;
@@ -2250,9 +2253,8 @@ int incident_run(fdtd_incident* b) {
     // them
     const IncidentBeam<T> beam = {r, (const T*)b->exc[0], (const T*)b->exc[1], b->feed_in, b->nt_pulse};
     T* const other[3] = {(T*)s->fld[1][3], (T*)s->fld[1][4], (T*)s->fld[1][5]};
-    done = launch_resident_beam<T>(st, other, beam, s->tdev, g.nt, (unsigned*)(s->tdev + 4), s->tdev + 6, s->stream);
-    if (done) s->wait_look = true;
-    else cudaGetLastError();   // a device without cooperative launches: single steps
+    done = launch_resident_beam<T>(st, other, beam, s->tdev, g.nt, (unsigned*)(s->tdev + 4), s->waited, s->stream);
+    if (!done) cudaGetLastError();   // a device without cooperative launches: single steps
   }
   if (done) {
   } else if (s->kernel == FDTD_KERNEL_FUSED) {
