@@ -83,6 +83,12 @@ extern "C" {
                                     advance several steps per launch, with the
                                     same results bit for bit (default 0). Not
                                     used while FDTD_OPT_CHECK_EVERY is on */
+#define FDTD_OPT_WAIT_LIMIT_US 14 /* longest wait, in us, of a resident launch's
+                                    blocks for one another (default 2000000, at
+                                    most 10 s). When it runs out the launch ends,
+                                    and every call that synchronises or hands
+                                    out results fails with FDTD_ERR_CUDA until
+                                    fdtd_reset */
 
 /* several steps per launch (fdtd_set_option(FDTD_OPT_MULTISTEP, ...)) */
 #define FDTD_MULTI_OFF      0
@@ -451,8 +457,8 @@ int fdtd_incident_create(const fdtd_geometry *geom, int nt_pulse, int device,
 int fdtd_incident_destroy(fdtd_incident *inc);
 /* FDTD_OPT_KERNEL (default FDTD_KERNEL_FUSED: the fused step, its source
  * plane written after each step), FDTD_OPT_TILE_Y, FDTD_OPT_ZCHUNK,
- * FDTD_OPT_FUSED_SLAB, FDTD_OPT_MULTISTEP (here default FDTD_MULTI_AUTO:
- * grids that stay in L2 run all steps in one launch; no pairs). */
+ * FDTD_OPT_FUSED_SLAB, FDTD_OPT_WAIT_LIMIT_US, FDTD_OPT_MULTISTEP (here default
+ * FDTD_MULTI_AUTO: grids that stay in L2 run all steps in one launch; no pairs). */
 int fdtd_incident_set_option(fdtd_incident *inc, int option, int value);
 /* 8 * npml profiles, packed as for fdtd_set_absorbers (Absorbers(params)
  * of the incident simulation, cpu/fdtd_sim.py:14-23). */

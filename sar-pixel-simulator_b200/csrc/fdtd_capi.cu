@@ -130,6 +130,7 @@ struct fdtd_sim {
   // this grid or no memory for it), its plan and tensor maps (one set per
   // source set), a third stream for its z-face chunks
   int multi = 0;
+  int wait_us = 2000000;                 // FDTD_OPT_WAIT_LIMIT_US
   bool side_by_side = false;             // running among a batch's streams
   int pair_state = 0;
   PairPlan pair;
@@ -141,7 +142,7 @@ struct fdtd_sim {
   // with the settings they were captured under; absorber uploads bump the
   // epoch (the profiles are captured by value)
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  int gsig[2][10] = {};
+  int gsig[2][11] = {};
   int gend[2] = {};                      // the current set after a replay
   int graph_epoch = 0;
   // gradient (fdtd_grad_*): checkpoints of the forward solve, the segment
@@ -235,13 +236,12 @@ int take_bounds_violation() {
               n, bytes, what, line);
 }
 
-// A wait inside a kernel that ran out since the last look (the results of
-// that run are not valid). After a synchronisation of the handle's stream.
-int take_wait_error(fdtd_sim* s) {
-  volatile int* w = s->waited;
-  if (!*w) return FDTD_OK;
-  *w = 0;
-  return fail(FDTD_ERR_CUDA, "a wait inside a step kernel ran out: the run's results are not valid");
+// A wait inside a kernel that ran out since the last reset: what the handle
+// holds is not valid, and every call that hands it out says so. After a
+// synchronisation of the handle's stream.
+int wait_error(const fdtd_sim* s) {
+  if (!*(const volatile int*)s->waited) return FDTD_OK;
+  return fail(FDTD_ERR_CUDA, "a wait inside a step kernel ran out: the results are not valid (fdtd_reset)");
 }
 
 void release(fdtd_sim* s, void* p) {
@@ -474,6 +474,8 @@ bool takes_pair(const fdtd_sim* s) {
          (s->esz == 8 ? cells >= kPairCellsDouble : cells >= kPairCellsFloat && s->g.nx >= kPairNxFloat);
 }
 
+unsigned long long wait_ns(const fdtd_sim* s) { return 1000ull * (unsigned long long)s->wait_us; }
+
 template <class T>
 int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
   if (takes_resident<T>(s, n)) {
@@ -484,7 +486,7 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     mark(s, e0);
     T* const other[3] = {(T*)s->fld[1 - s->cur][3], (T*)s->fld[1 - s->cur][4], (T*)s->fld[1 - s->cur][5]};
     const bool ok = launch_resident<T>(make_state<T>(s, s->cur, s->cur), other, s->tdev, 0, n, ph_g0, ph_ng,
-                                       (unsigned*)(s->tdev + 4), s->waited, s->stream);
+                                       (unsigned*)(s->tdev + 4), s->waited, wait_ns(s), s->stream);
     mark(s, e1);
     mark(s, e2);
     if (ok) {
@@ -591,8 +593,8 @@ template <class T>
 int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
   const int start = s->cur;
   if (takes_pair(s)) pair_ready<T>(s);   // allocates: not during a capture
-  const int sig[10] = {chunk,          s->kernel,      s->tile_x, s->tile_y, s->zchunk,
-                       s->phasor_mode, s->graph_epoch, s->slab,   s->shell,  s->multi};
+  const int sig[11] = {chunk,          s->kernel,      s->tile_x, s->tile_y, s->zchunk, s->phasor_mode,
+                       s->graph_epoch, s->slab,        s->shell,  s->multi,  s->wait_us};
   if (!s->gexec[start] || memcmp(sig, s->gsig[start], sizeof(sig)) != 0) {
     if (s->gexec[start]) {
       cudaGraphExecDestroy(s->gexec[start]);
@@ -917,6 +919,10 @@ int fdtd_set_option(fdtd_sim* s, int option, int value) {
         return fail(FDTD_ERR_INVALID, "unknown multi-step mode %d", value);
       s->multi = value;
       return FDTD_OK;
+    case FDTD_OPT_WAIT_LIMIT_US:
+      if (value < 0 || value > 10000000) return fail(FDTD_ERR_INVALID, "wait limit of %d us outside [0, 10 s]", value);
+      s->wait_us = value;
+      return FDTD_OK;
   }
   return fail(FDTD_ERR_INVALID, "unknown option %d", option);
 }
@@ -935,6 +941,7 @@ int fdtd_get_option(fdtd_sim* s, int option, int* value) {
     case FDTD_OPT_CHECK_EVERY: *value = s->check_every; return FDTD_OK;
     case FDTD_OPT_TIMING: *value = s->timing; return FDTD_OK;
     case FDTD_OPT_MULTISTEP: *value = s->multi; return FDTD_OK;
+    case FDTD_OPT_WAIT_LIMIT_US: *value = s->wait_us; return FDTD_OK;
   }
   return fail(FDTD_ERR_INVALID, "unknown option %d", option);
 }
@@ -1284,7 +1291,7 @@ int fdtd_synchronize(fdtd_sim* s) {
   CK(cudaStreamSynchronize(s->stream));
   CK(cudaGetLastError());
   if ((rc = take_bounds_violation())) return rc;
-  if ((rc = take_wait_error(s))) return rc;
+  if ((rc = wait_error(s))) return rc;
   if (s->check_every > 0) {
     int f[2] = {0, 0};
     CK(cudaMemcpy(f, s->flags, sizeof(f), cudaMemcpyDeviceToHost));
@@ -1349,7 +1356,7 @@ int fdtd_get_phasor(fdtd_sim* s, int plane, void* out) {
   CK(cudaMemcpyAsync(out, (char*)s->ph + s->ph_off[plane] * s->esz, (size_t)(2 * n) * s->esz,
                      cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  return take_wait_error(s);
+  return wait_error(s);
 }
 
 int fdtd_get_phasors(fdtd_sim* s, void* out) {
@@ -1369,7 +1376,7 @@ int fdtd_get_phasors(fdtd_sim* s, void* out) {
     off += bytes;
   }
   CK(cudaStreamSynchronize(s->stream));
-  return take_wait_error(s);
+  return wait_error(s);
 }
 
 int fdtd_get_field(fdtd_sim* s, int comp, void* out) {
@@ -1382,7 +1389,7 @@ int fdtd_get_field(fdtd_sim* s, int comp, void* out) {
   CK(cudaMemcpy2DAsync(out, w, s->fld[s->cur][comp], (size_t)s->pitch * s->esz, w,
                        (size_t)s->g.ny * s->g.nz, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  return take_wait_error(s);
+  return wait_error(s);
 }
 
 int fdtd_set_field(fdtd_sim* s, int comp, const void* in) {
@@ -1893,7 +1900,7 @@ int fdtd_batch_synchronize(fdtd_batch* b) {
   CK(cudaStreamSynchronize(b->stream));
   CK(cudaGetLastError());
   for (fdtd_sim* s : b->sims) {
-    const int rc = take_wait_error(s);
+    const int rc = wait_error(s);
     if (rc) return rc;
   }
   return take_bounds_violation();
@@ -1930,7 +1937,8 @@ int fdtd_near_field_power(fdtd_sim* s, const void* inc_phasors, int size_z_mater
     cudaError_t ce = cudaGetLastError();
     return fail(FDTD_ERR_CUDA, "near-field power: %s", cudaGetErrorString(ce));
   }
-  return take_bounds_violation();
+  if ((rc = take_bounds_violation())) return rc;
+  return wait_error(s);
 }
 
 int fdtd_batch_get_stream(fdtd_batch* b, void** stream) {
@@ -2140,6 +2148,7 @@ int fdtd_grad_forward(fdtd_sim* s, int checkpoint_every) {
     s->t += n;
   }
   CK(cudaStreamSynchronize(s->stream));
+  if ((rc = wait_error(s))) return rc;
   s->grad_forward_done = true;
   return FDTD_OK;
 }
@@ -2223,6 +2232,7 @@ template <class T>
 int incident_run(fdtd_incident* b) {
   fdtd_sim* s = b->sim;
   const fdtd_geometry& g = s->g;
+  b->ran = false;   // until this run is through
   int rc = fdtd_reset(s);
   if (rc) return rc;
   const size_t phb = (size_t)8 * s->ny_ph * s->nx_ph * s->esz;
@@ -2253,7 +2263,8 @@ int incident_run(fdtd_incident* b) {
     // them
     const IncidentBeam<T> beam = {r, (const T*)b->exc[0], (const T*)b->exc[1], b->feed_in, b->nt_pulse};
     T* const other[3] = {(T*)s->fld[1][3], (T*)s->fld[1][4], (T*)s->fld[1][5]};
-    done = launch_resident_beam<T>(st, other, beam, s->tdev, g.nt, (unsigned*)(s->tdev + 4), s->waited, s->stream);
+    done = launch_resident_beam<T>(st, other, beam, s->tdev, g.nt, (unsigned*)(s->tdev + 4), s->waited,
+                                   wait_ns(s), s->stream);
     if (!done) cudaGetLastError();   // a device without cooperative launches: single steps
   }
   if (done) {
@@ -2282,7 +2293,7 @@ int incident_run(fdtd_incident* b) {
   }
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(s->stream));
-  if ((rc = take_wait_error(s))) return rc;
+  if ((rc = wait_error(s))) return rc;
   s->t = g.nt;
   b->ran = true;
   return FDTD_OK;
@@ -2394,7 +2405,7 @@ int fdtd_incident_set_option(fdtd_incident* b, int option, int value) {
   int rc = check_inc(b);
   if (rc) return rc;
   if (option != FDTD_OPT_KERNEL && option != FDTD_OPT_TILE_Y && option != FDTD_OPT_ZCHUNK &&
-      option != FDTD_OPT_FUSED_SLAB && option != FDTD_OPT_MULTISTEP)
+      option != FDTD_OPT_FUSED_SLAB && option != FDTD_OPT_MULTISTEP && option != FDTD_OPT_WAIT_LIMIT_US)
     return fail(FDTD_ERR_INVALID, "option %d does not apply to an incident run", option);
   return fdtd_set_option(b->sim, option, value);
 }

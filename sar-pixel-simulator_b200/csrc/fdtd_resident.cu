@@ -34,8 +34,6 @@ namespace fdtd {
 
 namespace {
 
-constexpr unsigned long long kBarrierNs = 2000000000ull;
-
 // Kinds of boundary terms (fdtd_vecn.cuh): everything, and nothing.
 struct ResAll {
   static constexpr bool kX = true, kY = true, kZ = true;
@@ -55,8 +53,9 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 // All blocks of the launch have arrived `turn` times. sync[0] counts
-// arrivals, sync[1] is set when a wait ran out. False: give up.
-__device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned turn) {
+// arrivals, sync[1] is set when a wait ran out of its limit_ns. False: give
+// up.
+__device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned turn, unsigned long long limit_ns) {
   __shared__ int go;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -70,7 +69,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned turn) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(sync) : "memory");
       if (n >= want) break;
       const unsigned long long now = global_ns();
-      if (!end) end = now + kBarrierNs;
+      if (!end) end = now + limit_ns;
       if (now > end || *(volatile unsigned*)(sync + 1)) {
         atomicExch(sync + 1, 1u);
         ok = 0;
@@ -166,7 +165,7 @@ k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp
     if (n > 0) phasors(hs, t - 1);
     if constexpr (kBeam)
       read_out([&](int y, int x) { inc_record_e<T>(a.beam.rec, s.iex, s.iey, t, y, x); });
-    if (in_place && n > 0 && !grid_barrier(sync, ++turn)) break;
+    if (in_place && n > 0 && !grid_barrier(sync, ++turn, a.wait_ns)) break;
     sweep([&](int z, const PairPos<T, V>& p, unsigned i, bool easy) {
       T ph[6][V], pe[6][V];
       if (!easy) pair_psi<ResAll, 1>(s, p, z, ph, pe, load);
@@ -184,7 +183,7 @@ k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp
       stg(hd[0] + i, hx); stg(hd[1] + i, hy); stg(hd[2] + i, hz);
       if (!easy) pair_psi<ResAll, 1>(s, p, z, ph, pe, store);
     });
-    if (!grid_barrier(sync, ++turn)) break;
+    if (!grid_barrier(sync, ++turn, a.wait_ns)) break;
     if constexpr (kBeam)
       read_out([&](int y, int x) { inc_record_h<T>(a.beam.rec, hd[0], hd[1], t, y, x); });
     sweep([&](int z, const PairPos<T, V>& p, unsigned i, bool easy) {
@@ -214,7 +213,7 @@ k_resident(const __grid_constant__ ResidentArgs<T> a, const int* __restrict__ tp
       stg(s.oex + i, ex); stg(s.oey + i, ey); stg(s.oez + i, ez);
       if (!easy) pair_psi<ResAll, 2>(s, p, z, ph, pe, store);
     });
-    if (!grid_barrier(sync, ++turn)) break;
+    if (!grid_barrier(sync, ++turn, a.wait_ns)) break;
     if (n == nsteps - 1) phasors(cur, t);
   }
   if (threadIdx.x == 0 && *(volatile unsigned*)(sync + 1)) *err = 1;
@@ -290,28 +289,29 @@ bool resident(ResidentArgs<T>& a, const State<T>& s, T* const other_h[3], const 
 
 template <class T>
 bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, int toff, int nsteps, int ph_g0,
-                     int ph_ng, unsigned* sync, int* err, cudaStream_t st) {
+                     int ph_ng, unsigned* sync, int* err, unsigned long long wait_ns, cudaStream_t st) {
   ResidentArgs<T> a;
   memset(&a, 0, sizeof(a));
+  a.wait_ns = wait_ns;
   return resident<T, false>(a, s, other_h, tdev, toff, nsteps, ph_g0, ph_ng, sync, err, st);
 }
 
 template <class T>
 bool launch_resident_beam(const State<T>& s, T* const other_h[3], const IncidentBeam<T>& beam, const int* tdev,
-                          int nsteps, unsigned* sync, int* err, cudaStream_t st) {
+                          int nsteps, unsigned* sync, int* err, unsigned long long wait_ns, cudaStream_t st) {
   ResidentArgs<T> a;
   memset(&a, 0, sizeof(a));
   a.beam = beam;
+  a.wait_ns = wait_ns;
   return resident<T, true>(a, s, other_h, tdev, 0, nsteps, 0, 0, sync, err, st);
 }
 
-template bool launch_resident_beam<float>(const State<float>&, float* const[3], const IncidentBeam<float>&, const int*,
-                                          int, unsigned*, int*, cudaStream_t);
-template bool launch_resident_beam<double>(const State<double>&, double* const[3], const IncidentBeam<double>&,
-                                           const int*, int, unsigned*, int*, cudaStream_t);
-template bool launch_resident<float>(const State<float>&, float* const[3], const int*, int, int, int, int, unsigned*,
-                                     int*, cudaStream_t);
-template bool launch_resident<double>(const State<double>&, double* const[3], const int*, int, int, int, int,
-                                      unsigned*, int*, cudaStream_t);
+#define FDTD_RESIDENT_INSTANCES(T)                                                                                \
+  template bool launch_resident_beam<T>(const State<T>&, T* const[3], const IncidentBeam<T>&, const int*, int,    \
+                                        unsigned*, int*, unsigned long long, cudaStream_t);                       \
+  template bool launch_resident<T>(const State<T>&, T* const[3], const int*, int, int, int, int, unsigned*, int*, \
+                                   unsigned long long, cudaStream_t);
+FDTD_RESIDENT_INSTANCES(float)
+FDTD_RESIDENT_INSTANCES(double)
 
 }  // namespace fdtd

@@ -52,6 +52,7 @@ MULTI_OFF = 0
 MULTI_AUTO = 1
 MULTI_RESIDENT = 2
 MULTI_PAIR = 3
+OPT_WAIT_LIMIT_US = 14
 BATCH_SPLIT = 0
 BATCH_STREAMS = 1
 BATCH_QUEUE = 2
