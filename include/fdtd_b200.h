@@ -89,6 +89,15 @@ extern "C" {
                                     and every call that synchronises or hands
                                     out results fails with FDTD_ERR_CUDA until
                                     fdtd_reset */
+#define FDTD_OPT_STEP_PATH    15 /* read only: the FDTD_PATH_* bits of the steps
+                                    that the last fdtd_run, fdtd_run_streamed,
+                                    fdtd_grad_forward or batch in streams mode
+                                    took on this handle (0: another batch mode) */
+
+/* step paths (fdtd_get_option(FDTD_OPT_STEP_PATH, ...)) */
+#define FDTD_PATH_SINGLE    1
+#define FDTD_PATH_RESIDENT  2
+#define FDTD_PATH_PAIR      4
 
 /* several steps per launch (fdtd_set_option(FDTD_OPT_MULTISTEP, ...)) */
 #define FDTD_MULTI_OFF      0

@@ -144,6 +144,8 @@ struct fdtd_sim {
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   int gsig[2][11] = {};
   int gend[2] = {};                      // the current set after a replay
+  int gpath[2] = {};                     // the paths it holds
+  int path = 0;                          // FDTD_OPT_STEP_PATH: those of the last run
   int graph_epoch = 0;
   // gradient (fdtd_grad_*): checkpoints of the forward solve, the segment
   // of recomputed states and the adjoint state; a state is the 6 fields
@@ -490,6 +492,7 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     mark(s, e1);
     mark(s, e2);
     if (ok) {
+      s->path |= FDTD_PATH_RESIDENT;
       launch_advance(s->tdev, n, s->stream);
       CK(cudaGetLastError());
       return FDTD_OK;
@@ -515,11 +518,13 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     if (takes_pair(s) && k + 2 <= n && pair_ready<T>(s)) {
       const int rc = enqueue_pair<T>(s, k, ph_g0, ph_ng, e1);
       if (rc) return rc;
+      s->path |= FDTD_PATH_PAIR;
       mark(s, e2);
       if (s->timing) s->ev_steps.back() = 2;
       ++k;
       continue;
     }
+    s->path |= FDTD_PATH_SINGLE;
     if (s->kernel == FDTD_KERNEL_FUSED) {
       const int nxt = 1 - s->cur;
       if (!fused_supported_tile(s->tile_x, s->tile_y, (int)sizeof(T)))
@@ -601,9 +606,13 @@ int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
       s->gexec[start] = nullptr;
     }
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    const int before = s->path;
+    s->path = 0;
     const int rc = enqueue_steps<T>(s, chunk);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
+    s->gpath[start] = s->path;
+    s->path = before;
     s->gend[start] = s->cur;
     s->cur = start;   // capturing ran nothing
     if (rc || e != cudaSuccess) {
@@ -620,6 +629,7 @@ int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
     memcpy(s->gsig[start], sig, sizeof(sig));
   }
   CK(cudaGraphLaunch(s->gexec[start], s->stream));
+  s->path |= s->gpath[start];
   s->cur = s->gend[start];
   return FDTD_OK;
 }
@@ -629,6 +639,7 @@ int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
 // absolute step) is on, direct launches otherwise and for the remainder.
 template <class T>
 int run_steps(fdtd_sim* s, int nsteps) {
+  s->path = 0;
   const int chunk = s->graph_chunk;
   if (chunk > 0 && !s->timing && s->check_every == 0) {
     while (nsteps >= chunk) {
@@ -923,6 +934,8 @@ int fdtd_set_option(fdtd_sim* s, int option, int value) {
       if (value < 0 || value > 10000000) return fail(FDTD_ERR_INVALID, "wait limit of %d us outside [0, 10 s]", value);
       s->wait_us = value;
       return FDTD_OK;
+    case FDTD_OPT_STEP_PATH:
+      return fail(FDTD_ERR_INVALID, "FDTD_OPT_STEP_PATH is read only");
   }
   return fail(FDTD_ERR_INVALID, "unknown option %d", option);
 }
@@ -942,6 +955,7 @@ int fdtd_get_option(fdtd_sim* s, int option, int* value) {
     case FDTD_OPT_TIMING: *value = s->timing; return FDTD_OK;
     case FDTD_OPT_MULTISTEP: *value = s->multi; return FDTD_OK;
     case FDTD_OPT_WAIT_LIMIT_US: *value = s->wait_us; return FDTD_OK;
+    case FDTD_OPT_STEP_PATH: *value = s->path; return FDTD_OK;
   }
   return fail(FDTD_ERR_INVALID, "unknown option %d", option);
 }
@@ -1246,6 +1260,7 @@ int fdtd_run_streamed(fdtd_sim* s, int nsteps, const void* ex, const void* ey, c
     if (alloc(s, 2 * dslot, &s->dstage) == FDTD_OK) s->dstage_bytes = 2 * dslot;
   }
   cudaGetLastError();
+  s->path = 0;
   // the first group is short, so that the stepping starts early
   for (int c0 = t0, slot = 0, grp = std::min(2, chunk); c0 < t1; c0 += grp, slot ^= 1, grp = chunk) {
     const int n = std::min(grp, t1 - c0);
@@ -1571,6 +1586,7 @@ int batch_run(fdtd_batch* b, int nsteps) {
   for (fdtd_sim* s : b->sims) {
     CK(cudaStreamWaitEvent(s->stream, b->ev, 0));
     s->t += nsteps;
+    s->path = 0;
   }
   return FDTD_OK;
 }
@@ -1751,6 +1767,7 @@ int batch_run_queue(fdtd_batch* b, int nsteps) {
   for (fdtd_sim* s : b->sims) {
     CK(cudaStreamWaitEvent(s->stream, b->ev, 0));
     s->t += nsteps;
+    s->path = 0;
     if (nsteps & 1) s->cur = 1 - s->cur;
   }
   return FDTD_OK;
@@ -2139,6 +2156,7 @@ int fdtd_grad_forward(fdtd_sim* s, int checkpoint_every) {
   s->grad_ncp = ncp;
   s->grad_forward_done = false;
   if ((rc = fdtd_reset(s))) return rc;
+  s->path = 0;
   for (int c = 0; c < ncp; ++c) {
     if ((rc = save_state(s, static_cast<unsigned char*>(s->grad_cp) + c * sb))) return rc;
     const int n = std::min(checkpoint_every, nt - c * checkpoint_every);

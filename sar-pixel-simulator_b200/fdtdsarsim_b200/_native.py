@@ -53,6 +53,10 @@ MULTI_AUTO = 1
 MULTI_RESIDENT = 2
 MULTI_PAIR = 3
 OPT_WAIT_LIMIT_US = 14
+OPT_STEP_PATH = 15
+PATH_SINGLE = 1
+PATH_RESIDENT = 2
+PATH_PAIR = 4
 BATCH_SPLIT = 0
 BATCH_STREAMS = 1
 BATCH_QUEUE = 2
