@@ -142,7 +142,7 @@ struct fdtd_sim {
   // with the settings they were captured under; absorber uploads bump the
   // epoch (the profiles are captured by value)
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  int gsig[2][11] = {};
+  int gsig[2][12] = {};
   int gend[2] = {};                      // the current set after a replay
   int gpath[2] = {};                     // the paths it holds
   int path = 0;                          // FDTD_OPT_STEP_PATH: those of the last run
@@ -598,8 +598,10 @@ template <class T>
 int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
   const int start = s->cur;
   if (takes_pair(s)) pair_ready<T>(s);   // allocates: not during a capture
-  const int sig[11] = {chunk,          s->kernel,      s->tile_x, s->tile_y, s->zchunk, s->phasor_mode,
-                       s->graph_epoch, s->slab,        s->shell,  s->multi,  s->wait_us};
+  // a resident run among a batch's streams takes single steps: the choice is
+  // part of what was captured
+  const int sig[12] = {chunk,          s->kernel, s->tile_x, s->tile_y, s->zchunk,  s->phasor_mode,
+                       s->graph_epoch, s->slab,   s->shell,  s->multi,  s->wait_us, takes_resident<T>(s, chunk)};
   if (!s->gexec[start] || memcmp(sig, s->gsig[start], sizeof(sig)) != 0) {
     if (s->gexec[start]) {
       cudaGraphExecDestroy(s->gexec[start]);
