@@ -105,9 +105,12 @@ extern "C" {
 #define FDTD_MULTI_RESIDENT 2 /* every step of fdtd_run in one cooperative
                                  launch (not among a batch's streams) */
 #define FDTD_MULTI_PAIR     3 /* two steps per pass over the fields; holds a
-                                 few planes more (single steps where there is
-                                 no memory for them, or the grid is too
-                                 narrow) */
+                                 few planes more, allocated on the first run
+                                 (single steps where there is no memory for
+                                 them, where the caller captures that run, or
+                                 on a grid that gives no plain box of 32
+                                 columns and 8 rows inside the faces; with
+                                 npml above 10 none does) */
 
 /* batched sweep (fdtd_batch_set_option(FDTD_OPT_BATCH_MODE, ...)) */
 #define FDTD_BATCH_SPLIT   0   /* (default) one launch per pass (H, E, phasors)

@@ -378,10 +378,14 @@ int collect_timing(fdtd_sim* s) {
 
 // What the pair step needs beyond two field sets, made on first use: the
 // mid planes, the plan and maps. A grid without a column worth marching, or
-// a device without room, takes single steps.
+// a device without room, takes single steps; so does a caller's capture of
+// the first run, in which nothing can be allocated (a later run is asked
+// again).
 template <class T>
 bool pair_ready(fdtd_sim* s) {
   if (s->pair_state) return s->pair_state > 0;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
   s->pair_state = -1;
   const fdtd_geometry& g = s->g;
   s->pair = make_pair_plan(g.nx, g.ny, g.nz, g.npml, (int)sizeof(T));
