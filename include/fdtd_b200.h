@@ -102,8 +102,10 @@ extern "C" {
 /* several steps per launch (fdtd_set_option(FDTD_OPT_MULTISTEP, ...)) */
 #define FDTD_MULTI_OFF      0
 #define FDTD_MULTI_AUTO     1 /* by the grid's size: resident, pair or single */
-#define FDTD_MULTI_RESIDENT 2 /* every step of fdtd_run in one cooperative
-                                 launch (not among a batch's streams) */
+#define FDTD_MULTI_RESIDENT 2 /* many steps per cooperative launch (not among
+                                 a batch's streams). A launch holds every SM
+                                 for about a millisecond; work of other
+                                 streams and handles runs between launches */
 #define FDTD_MULTI_PAIR     3 /* two steps per pass over the fields; holds a
                                  few planes more, allocated on the first run
                                  (single steps where there is no memory for
@@ -470,7 +472,7 @@ int fdtd_incident_destroy(fdtd_incident *inc);
 /* FDTD_OPT_KERNEL (default FDTD_KERNEL_FUSED: the fused step, its source
  * plane written after each step), FDTD_OPT_TILE_Y, FDTD_OPT_ZCHUNK,
  * FDTD_OPT_FUSED_SLAB, FDTD_OPT_WAIT_LIMIT_US, FDTD_OPT_MULTISTEP (here default
- * FDTD_MULTI_AUTO: grids that stay in L2 run all steps in one launch; no pairs). */
+ * FDTD_MULTI_AUTO: grids that stay in L2 run many steps per launch; no pairs). */
 int fdtd_incident_set_option(fdtd_incident *inc, int option, int value);
 /* 8 * npml profiles, packed as for fdtd_set_absorbers (Absorbers(params)
  * of the incident simulation, cpu/fdtd_sim.py:14-23). */

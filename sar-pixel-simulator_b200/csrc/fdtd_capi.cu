@@ -480,6 +480,16 @@ bool takes_pair(const fdtd_sim* s) {
          (s->esz == 8 ? cells >= kPairCellsDouble : cells >= kPairCellsFloat && s->g.nx >= kPairNxFloat);
 }
 
+// Steps of each resident launch of a run of n: about a millisecond, because a
+// launch holds every SM and the work of other streams and handles waits for its
+// end (even: the launch then never updates H in place). A step takes about
+// 7 us and 1 us per 150 KB of one field (the sizes above).
+int resident_launch_steps(const fdtd_sim* s, int n) {
+  const double us = 7.0 + (double)s->vol * s->esz / 150e3;
+  const int most = std::max(2, (int)(1000.0 / us)), launches = (n + most - 1) / most;
+  return ((n + launches - 1) / launches + 1) & ~1;
+}
+
 unsigned long long wait_ns(const fdtd_sim* s) { return 1000ull * (unsigned long long)s->wait_us; }
 
 template <class T>
@@ -491,11 +501,18 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     if (s->timing) s->ev_steps.push_back(n);
     mark(s, e0);
     T* const other[3] = {(T*)s->fld[1 - s->cur][3], (T*)s->fld[1 - s->cur][4], (T*)s->fld[1 - s->cur][5]};
-    const bool ok = launch_resident<T>(make_state<T>(s, s->cur, s->cur), other, s->tdev, 0, n, ph_g0, ph_ng,
-                                       (unsigned*)(s->tdev + 4), s->waited, wait_ns(s), s->stream);
+    const State<T> st = make_state<T>(s, s->cur, s->cur);
+    const int each = resident_launch_steps(s, n);
+    int done = 0;
+    while (done < n &&
+           launch_resident<T>(st, other, s->tdev, done, std::min(each, n - done), ph_g0, ph_ng,
+                              (unsigned*)(s->tdev + 4), s->waited, wait_ns(s), s->stream))
+      done += std::min(each, n - done);
     mark(s, e1);
     mark(s, e2);
-    if (ok) {
+    if (done > 0 && done < n)
+      return fail(FDTD_ERR_CUDA, "resident step launch: %s", cudaGetErrorString(cudaGetLastError()));
+    if (done == n) {
       s->path |= FDTD_PATH_RESIDENT;
       launch_advance(s->tdev, n, s->stream);
       CK(cudaGetLastError());
@@ -2283,12 +2300,17 @@ int incident_run(fdtd_incident* b) {
   source(0, 0);
   bool done = false;
   if (takes_resident<T>(s, g.nt)) {
-    // every step in one resident launch, the source and the read-out with
-    // them
+    // resident launches, the source and the read-out with the steps
     const IncidentBeam<T> beam = {r, (const T*)b->exc[0], (const T*)b->exc[1], b->feed_in, b->nt_pulse};
     T* const other[3] = {(T*)s->fld[1][3], (T*)s->fld[1][4], (T*)s->fld[1][5]};
-    done = launch_resident_beam<T>(st, other, beam, s->tdev, g.nt, (unsigned*)(s->tdev + 4), s->waited,
-                                   wait_ns(s), s->stream);
+    const int each = resident_launch_steps(s, g.nt);
+    int t = 0;
+    while (t < g.nt && launch_resident_beam<T>(st, other, beam, s->tdev, t, std::min(each, g.nt - t),
+                                               (unsigned*)(s->tdev + 4), s->waited, wait_ns(s), s->stream))
+      t += std::min(each, g.nt - t);
+    done = t == g.nt;
+    if (t > 0 && !done)
+      return fail(FDTD_ERR_CUDA, "resident step launch: %s", cudaGetErrorString(cudaGetLastError()));
     if (!done) cudaGetLastError();   // a device without cooperative launches: single steps
   }
   if (done) {

@@ -200,17 +200,19 @@ struct ResidentArgs {
 };
 // Enqueues nsteps steps from the step *tdev + toff (their phasors in plane
 // groups ph_g0 .. ph_g0 + ph_ng - 1 included); the run ends on the set it
-// began with. sync: two words of device memory; *err (host-mapped) is set when
-// a barrier waited longer than wait_ns. False: not launched.
+// began with. sync: two words of device memory, zero after a reset; *err
+// (host-mapped) is set when a barrier waited longer than wait_ns. False: not
+// launched.
 template <class T>
 bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, int toff, int nsteps, int ph_g0,
                      int ph_ng, unsigned* sync, int* err, unsigned long long wait_ns, cudaStream_t st);
-// The same for an incident run's steps 0 .. nsteps - 1, whose first E update
-// and source are done: each H update, then the next step's E update with its
-// source; the read-out plane of every step beside them.
+// The same for an incident run's steps toff .. toff + nsteps - 1, whose first
+// E update and source are done: each H update, then the next step's E update
+// with its source; the read-out plane of every step beside them.
 template <class T>
 bool launch_resident_beam(const State<T>& s, T* const other_h[3], const IncidentBeam<T>& beam, const int* tdev,
-                          int nsteps, unsigned* sync, int* err, unsigned long long wait_ns, cudaStream_t st);
+                          int toff, int nsteps, unsigned* sync, int* err, unsigned long long wait_ns,
+                          cudaStream_t st);
 
 // Pair step (fdtd_pair.cu): two steps per pass, by marches over regions of
 // four kinds. A region is the box x [x0, x1), y [y0, y1), z [z0, z1), cut

@@ -10,8 +10,10 @@
 // E and the CPML auxiliaries are updated in place; H alternates between two
 // sets, so that the phasors of the finished step can read its H beside the
 // H pass that follows. The last of an odd number of steps updates H in place
-// (after its predecessor's phasors), so that a run ends on the set it began
-// with. The updates are the split passes' (fdtd_split.cuh), bit for bit.
+// (after its predecessor's phasors), so that a launch ends on the set it began
+// with. A launch is of about a millisecond (resident_launch_steps,
+// fdtd_capi.cu), because it holds every SM: a run of one launch instead of
+// one per millisecond is 0.4 % to 0.9 % faster, but stops every other stream. The updates are the split passes' (fdtd_split.cuh), bit for bit.
 //
 // The barrier waits with a time limit, after which every block leaves and
 // the launch is reported as failed.
@@ -53,8 +55,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 // All blocks of the launch have arrived `turn` times. sync[0] counts
-// arrivals, sync[1] is set when a wait ran out of its limit_ns. False: give
-// up.
+// arrivals, sync[1] is set when a wait ran out of its limit_ns (cleared by a
+// reset of the handle). False: give up.
 __device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned turn, unsigned long long limit_ns) {
   __shared__ int go;
   __syncthreads();
@@ -259,7 +261,9 @@ bool resident_launch(ResidentArgs<T>& a, const int* tdev, int toff, int nsteps, 
   a.per_row = div_magic((unsigned)a.gx);
   a.per_plane = div_magic((unsigned)a.gy);
   void* args[] = {&a, &tdev, &toff, &nsteps, &ph_g0, &ph_ng, &sync, &err};
-  return cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), st) == cudaSuccess &&
+  // sync[1] stays: after a wait that ran out the launches that follow leave at
+  // their first barrier
+  return cudaMemsetAsync(sync, 0, sizeof(unsigned), st) == cudaSuccess &&
          cudaLaunchCooperativeKernel((const void*)k_resident<T, V, kBeam>, dim3(blocks), dim3(kResThreads<T, V>), args, 0,
                                      st) == cudaSuccess;
 }
@@ -298,17 +302,18 @@ bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, in
 
 template <class T>
 bool launch_resident_beam(const State<T>& s, T* const other_h[3], const IncidentBeam<T>& beam, const int* tdev,
-                          int nsteps, unsigned* sync, int* err, unsigned long long wait_ns, cudaStream_t st) {
+                          int toff, int nsteps, unsigned* sync, int* err, unsigned long long wait_ns,
+                          cudaStream_t st) {
   ResidentArgs<T> a;
   memset(&a, 0, sizeof(a));
   a.beam = beam;
   a.wait_ns = wait_ns;
-  return resident<T, true>(a, s, other_h, tdev, 0, nsteps, 0, 0, sync, err, st);
+  return resident<T, true>(a, s, other_h, tdev, toff, nsteps, 0, 0, sync, err, st);
 }
 
 #define FDTD_RESIDENT_INSTANCES(T)                                                                                \
   template bool launch_resident_beam<T>(const State<T>&, T* const[3], const IncidentBeam<T>&, const int*, int,    \
-                                        unsigned*, int*, unsigned long long, cudaStream_t);                       \
+                                        int, unsigned*, int*, unsigned long long, cudaStream_t);                  \
   template bool launch_resident<T>(const State<T>&, T* const[3], const int*, int, int, int, int, unsigned*, int*, \
                                    unsigned long long, cudaStream_t);
 FDTD_RESIDENT_INSTANCES(float)
