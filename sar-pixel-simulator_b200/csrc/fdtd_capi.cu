@@ -376,6 +376,11 @@ int collect_timing(fdtd_sim* s) {
   return FDTD_OK;
 }
 
+// At most 4096 timed groups wait for collection.
+int room_for_timing(fdtd_sim* s) {
+  return s->timing && s->ev_used + 3 > 3 * 4096 ? collect_timing(s) : FDTD_OK;
+}
+
 // What the pair step needs beyond two field sets, made on first use: the
 // mid planes, the plan and maps. A grid without a column worth marching, or
 // a device without room, takes single steps; so does a caller's capture of
@@ -495,6 +500,7 @@ unsigned long long wait_ns(const fdtd_sim* s) { return 1000ull * (unsigned long 
 template <class T>
 int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
   if (takes_resident<T>(s, n)) {
+    if (const int rc = room_for_timing(s)) return rc;
     cudaEvent_t e0 = s->timing ? timing_event(s) : nullptr;
     cudaEvent_t e1 = s->timing ? timing_event(s) : nullptr;
     cudaEvent_t e2 = s->timing ? timing_event(s) : nullptr;
@@ -525,10 +531,7 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     }
   }
   for (int k = 0; k < n; ++k) {
-    if (s->timing && s->ev_used + 3 > 3 * 4096) {
-      int rc = collect_timing(s);
-      if (rc) return rc;
-    }
+    if (const int rc = room_for_timing(s)) return rc;
     cudaEvent_t e0 = s->timing ? timing_event(s) : nullptr;
     cudaEvent_t e1 = s->timing ? timing_event(s) : nullptr;
     cudaEvent_t e2 = s->timing ? timing_event(s) : nullptr;
