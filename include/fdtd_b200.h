@@ -393,11 +393,12 @@ int fdtd_near_field_power(fdtd_sim *sim, const void *inc_phasors, int size_z_mat
 int fdtd_bounds_check_enabled(void);
 
 /* Diagnostic (no counterpart in the reference): the CPML terms divide by
- * the cell size with a correctly rounded reciprocal and one FMA correction
- * (Markstein's method) instead of an IEEE division. This runs both on the
- * device for every float bit pattern (FDTD_F32: 2^32 inputs) or for 2^30
- * sampled doubles (FDTD_F64) with divisor `cell_size` rounded to the type,
- * and returns how many inputs gave a result that differs in any bit. */
+ * the cell size through its reciprocal (float: one double product; double: one
+ * FMA correction, Markstein's method) instead of an IEEE division, with the
+ * same quotient for every input. This runs both on the device for every
+ * float bit pattern (FDTD_F32: 2^32 inputs) or for 2^30 sampled doubles
+ * (FDTD_F64) with divisor `cell_size` rounded to the type, and returns how
+ * many inputs gave a result that differs in any bit. */
 int fdtd_check_cell_division(int dtype, double cell_size, int device, int64_t *tested,
                              int64_t *mismatches);
 

@@ -6,6 +6,8 @@
 // kernels (fdtdsarsim/cpu/field_updates.py), which do not contract either.
 #pragma once
 
+#include <cmath>
+
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -64,7 +66,7 @@ struct State {
   long long plane;   // ny * pitch
   T db, dtm0, dte0dx, dx;
   T rdx;         // 1 / dx correctly rounded (host IEEE division)
-  double rdx64;  // the same in double
+  double rdx64;  // its reciprocal for div_const (div_reciprocal)
   T prof[8][kMaxPml];
   // field sets: src is read, dst is written (the same set for the in-place
   // split kernels; ping-pong sets for the fused kernel)
@@ -168,22 +170,28 @@ struct InteriorBox {
   int chunks0, chunks;   // chunks of the first range, of both ranges
 };
 
-// Correctly rounded u / d for d > 0, given r = 1 / d correctly rounded in
-// double. Used for the CPML terms (c * dE) / dx, whose divisor is the
-// constant cell size.
+// Correctly rounded u / d for d > 0, given r = div_reciprocal(d). Used for the
+// CPML terms (c * dE) / dx, whose divisor is the constant cell size.
 //
-// Floats: the double product u r is within 2^-52 of u / d, and the quotient
-// of two floats lies at least 2^-49 (relative) from every float rounding
-// boundary that it does not lie on; it lies on one only where d is a power of
-// two (the product is then exact) or, for a subnormal quotient, where
-// d >= 2. Its rounding to float is therefore the quotient's, for every u:
-// zeros keep their sign, infinities and NaN pass. Three instructions, no
-// range test and no branch, where Markstein's correction takes two products,
-// two FMAs, a range test and a branch per term, and below 2^-100, which the
-// faint front of a wave meets, the IEEE division. Measured: a 32-member
-// batch 1.35 ms per step with the correction, 1.31 so.
+// Floats: r is the smallest double not below 1 / d, so the double product
+// u r lies from 2^-53 below u / d to 2^-51 above (relative), and without its
+// last two bits within 2^-50. The quotient of two floats lies more than 2^-49
+// from every float rounding boundary that it does not lie on, so the
+// product's rounding to float is the quotient's. On a boundary (d a power of
+// two, or d >= 2 and a subnormal quotient) the product is at most two last
+// places above it, which the cleared bits take off, and the boundary itself
+// is rounded. So for every u: zeros keep their sign, infinities and NaN pass.
+// Four instructions, no range test and no branch, where Markstein's correction
+// takes two products, two FMAs, a range test and a branch per term, and below
+// 2^-100, which the faint front of a wave meets, the IEEE division. Measured:
+// a 32-member batch 1.35 ms per step with the correction, 1.31 so.
 __device__ __forceinline__ float div_const(float u, float, double r) {
-  return __double2float_rn(__dmul_rn((double)u, r));
+  const double q = __dmul_rn((double)u, r);
+  return __double2float_rn(__hiloint2double(__double2hiint(q), __double2loint(q) & ~3));
+}
+inline double div_reciprocal(float d) {
+  const double r = 1.0 / (double)d;
+  return std::fma(r, (double)d, -1.0) < 0.0 ? std::nextafter(r, INFINITY) : r;
 }
 
 // Doubles: Markstein's FMA correction (P. W. Markstein, "Computation of
@@ -193,6 +201,7 @@ __device__ __forceinline__ float div_const(float u, float, double r) {
 // RN(q0 + r (u - d q0)) is the correctly rounded quotient, as long as no step
 // leaves the normal range. |u| outside [2^-900, 2^900] takes the IEEE
 // division instead.
+inline double div_reciprocal(double d) { return 1.0 / d; }
 __device__ __forceinline__ double div_const(double u, double d, double r) {
   const double lo = 1.4708983551653345e-271, hi = 6.7986211919640936e+270;   // 2^-900, 2^900
   const double a = fabs(u);

@@ -81,11 +81,11 @@ extern "C" int fdtd_check_cell_division(int dtype, double cell_size, int device,
   unsigned long long n;
   if (dtype == FDTD_F32) {
     const float d = (float)cell_size;
-    const double r = 1.0 / (double)d;   // IEEE division on the host
+    const double r = div_reciprocal(d);
     n = 1ULL << 32;
     k_check_div_f<<<148 * 16, 256>>>(d, r, bad);
   } else {
-    const double r = 1.0 / cell_size;
+    const double r = div_reciprocal(cell_size);
     n = 1ULL << 30;
     k_check_div_d<<<148 * 16, 256>>>(cell_size, r, n, bad);
   }
