@@ -39,8 +39,9 @@ CANDIDATES = [
     (_native.FDTD_KERNEL_FUSED, 4, 0, 0, _SPLIT, _native.MULTI_PAIR),
 ]
 
-# cache entries measured with another candidate set are measured again
-_VERSION = 'v4'
+# cache entries measured with another candidate set, or by another time, are
+# measured again
+_VERSION = 'v5'
 
 
 def cache_path():
@@ -115,8 +116,9 @@ def autotune(geom, device=0, steps=6, candidates=None, save=True):
 
     The measurement uses vacuum coefficients, CPML profiles of ones and
     zeros and no incident beam: the step kernels' cost does not depend on the
-    values (the one value-dependent branch, the IEEE division of tiny CPML
-    terms, is taken by subnormal inputs only)."""
+    values (doubles outside [2^-900, 2^900] divide by another branch). A
+    candidate's time is its whole step, phasors included: a resident run has
+    them within its one launch, where no event tells them apart."""
     g = _native.Geometry()
     for name, _ in _native.Geometry._fields_:
         setattr(g, name, getattr(geom, name))
@@ -144,6 +146,7 @@ def autotune(geom, device=0, steps=6, candidates=None, save=True):
             sim.set_option(_native.OPT_TIMING, 1)
             sim.run(steps)
             ms, n = sim.kernel_time(_native.TIME_STEP)
+            ms += sim.kernel_time(_native.TIME_PHASOR)[0]
             sim.set_option(_native.OPT_TIMING, 0)
         except _native.FdtdError:
             continue
