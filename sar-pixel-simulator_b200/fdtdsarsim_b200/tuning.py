@@ -131,7 +131,7 @@ def autotune(geom, device=0, steps=6, candidates=None, save=True):
     ca = np.ones((g.nz, g.ny, g.nx), ft)
     cb = np.full((g.nz, g.ny, g.nx), g.dte0dx, ft)
     sim.set_materials(ca, cb)
-    timings = []
+    timings, ran = [], []
     for cand in (candidates or CANDIDATES):
         kernel, ty, zc, slab = cand[:4]
         shell = cand[4] if len(cand) > 4 else _MARCH
@@ -148,15 +148,20 @@ def autotune(geom, device=0, steps=6, candidates=None, save=True):
             ms, n = sim.kernel_time(_native.TIME_STEP)
             ms += sim.kernel_time(_native.TIME_PHASOR)[0]
             sim.set_option(_native.OPT_TIMING, 0)
+            path = sim.get_option(_native.OPT_STEP_PATH)
         except _native.FdtdError:
             continue
         timings.append((ms / max(n, 1), choice))
+        # a grid too narrow for pairs runs single steps in their place
+        if path & {_native.MULTI_RESIDENT: _native.PATH_RESIDENT,
+                   _native.MULTI_PAIR: _native.PATH_PAIR}.get(choice['multi'], _native.PATH_SINGLE):
+            ran.append(timings[-1])
     sim.close()
-    best = min(timings, key=lambda t: t[0])[1]
+    best_ms, best = min(ran or timings, key=lambda t: t[0])
     if save:
         path = cache_path()
         data = _load()
-        data[_key(geom, _device_name(device))] = dict(best, step_ms=min(t[0] for t in timings))
+        data[_key(geom, _device_name(device))] = dict(best, step_ms=best_ms)
         os.makedirs(os.path.dirname(path), exist_ok=True)
         tmp = path + '.tmp'
         with open(tmp, 'w') as fh:

@@ -75,3 +75,9 @@ RES, PAIR = FUSED4 + (_native.MULTI_RESIDENT,), FUSED4 + (_native.MULTI_PAIR,)
     ({RES: (0.076, 0.0), FUSED4 + (0,): (0.075, 0.011)}, _native.MULTI_RESIDENT)])
 def test_candidates_are_compared_by_the_whole_step(tune, times, want):
     assert tune(times)['multi'] == want
+
+
+def test_a_candidate_that_fell_back_is_not_taken_for_its_name(tune):
+    times = {PAIR: (0.080, 0.01), FUSED4 + (0,): (0.081, 0.01)}
+    assert tune(times)['multi'] == _native.MULTI_PAIR
+    assert tune(times, narrow=True)['multi'] == _native.MULTI_OFF
