@@ -81,3 +81,11 @@ def test_a_candidate_that_fell_back_is_not_taken_for_its_name(tune):
     times = {PAIR: (0.080, 0.01), FUSED4 + (0,): (0.081, 0.01)}
     assert tune(times)['multi'] == _native.MULTI_PAIR
     assert tune(times, narrow=True)['multi'] == _native.MULTI_OFF
+
+
+@pytest.mark.parametrize('multi', [RES, PAIR])
+def test_several_steps_per_pass_keep_the_fastest_single_step_beside_them(tune, multi):
+    fast = (FUSED, 8, 0, _native.SHELL_MARCH)
+    best = tune({multi: (0.05, 0.0), fast + (0,): (0.07, 0.01), FUSED4 + (0,): (0.08, 0.01)})
+    assert best == {'kernel': FUSED, 'tile_x': 32, 'tile_y': 8, 'zchunk': 0, 'slab': 0,
+                    'shell': _native.SHELL_MARCH, 'multi': multi[-1]}
