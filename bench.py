@@ -261,15 +261,16 @@ def job_rate(units, steps, ms, world):
     return world * units * steps / (ms / 1e3) / 1e6
 
 
-def run_launches(choice, steps):
-    """Kernel launches of one run of `steps` steps: resident steps, one launch
-    and the counter's; a pair of steps, one march of each of the four regions
-    and the phasors; otherwise step_launches a step, and the counter's."""
+def run_launches(choice, steps, path):
+    """Kernel launches of one run of `steps` steps that took `path`
+    (FDTD_OPT_STEP_PATH): resident steps, one launch (at least: one per
+    millisecond) and the counter's; a pair of steps, one march of each of the
+    four regions and the phasors; otherwise step_launches a step, and the
+    counter's."""
     from fdtdsarsim_b200 import _native
-    multi = choice.get('multi', _native.MULTI_OFF) if choice['kernel'] == _native.FDTD_KERNEL_FUSED else 0
-    if multi == _native.MULTI_RESIDENT:
+    if path & _native.PATH_RESIDENT:
         return 2
-    if multi == _native.MULTI_PAIR:
+    if path & _native.PATH_PAIR:
         return 5 * (steps // 2) + step_launches(choice) * (steps % 2) + 1
     return step_launches(choice) * steps + 1
 
@@ -363,7 +364,8 @@ def run_ours(a):
     ms = t_start.elapsed_time(t_end)
     ms_max = max_over_ranks(ms, world, 'cuda')
     value = job_rate(cells, a.steps, ms_max, world)
-    gpu_launches = run_launches(choice, a.steps)
+    path = sim.get_option(_native.OPT_STEP_PATH)
+    gpu_launches = run_launches(choice, a.steps, path)
 
     # live per-kernel timing for the roofline (separate pass, same state)
     sim.reset()
@@ -377,7 +379,7 @@ def run_ours(a):
     ph_ms, ph_n = sim.kernel_time(_native.TIME_PHASOR)
     sim.set_option(_native.OPT_TIMING, 0)
     # a launch: one step, or one pass over the fields that makes two
-    per_pass = 2 if multi_name(choice) == 'pair' else 1
+    per_pass = 2 if path & _native.PATH_PAIR else 1
     kname = 'pair_step' if per_pass == 2 else \
         'fused_step' if choice['kernel'] == _native.FDTD_KERNEL_FUSED else 'split_h_e'
     avg_ms = per_pass * step_ms / max(step_n, 1)
@@ -569,9 +571,7 @@ def batch_record(a, n_models, steps, warmup, check_members=(0, 21, 42)):
         sim = _native.NativeSim(geom, 0)
         sim.set_absorbers(packed_profiles(pc))
         choice = tuning.choose(geom)
-        # side by side, the default's choice is between pairs and single steps
-        pairs = choice.get('multi') == _native.MULTI_AUTO and tuning.pair_pays(geom)
-        choices.append(dict(choice, multi=_native.MULTI_PAIR if pairs else choice.get('multi', 0)))
+        choices.append(choice)
         tuning.apply(sim, choice)
         sim.set_materials(ca, cb)
         sim.set_incident(inc['ex'], inc['ey'], inc['hx'], inc['hy'])
@@ -608,6 +608,7 @@ def batch_record(a, n_models, steps, warmup, check_members=(0, 21, 42)):
     batch.run(warmup)
     batch.synchronize()
     ms_streams = timed(bstream, lambda: batch.run(steps))
+    paths = [s.get_option(_native.OPT_STEP_PATH) for s in sims]
     snap_streams = snapshot()
     for s in sims:
         s.reset()
@@ -671,7 +672,7 @@ def batch_record(a, n_models, steps, warmup, check_members=(0, 21, 42)):
                      'kernel': {'streams': 'fused_step (member streams)', 'split': 'batch_split_step',
                                 'queue': 'batch_queue'}[mode]},
         'cpu_baseline': None, 'e2e': None,
-        'gpu_launches': {'streams': sum(run_launches(c, steps) for c in choices),
+        'gpu_launches': {'streams': sum(run_launches(c, steps, p) for c, p in zip(choices, paths)),
                          'split': 3 * steps + 1,
                          'queue': 2 * steps + 1}[mode],
         'clocks': clk,

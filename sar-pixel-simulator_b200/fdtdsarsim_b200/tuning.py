@@ -91,13 +91,6 @@ def choose(geom, kernel=None, tile=None, device=0, use_cache=True):
             'multi': _native.MULTI_AUTO if kernel is None and tile is None else _native.MULTI_OFF}
 
 
-def pair_pays(geom):
-    """Whether MULTI_AUTO takes two steps per pass on this grid (where it does
-    not run them resident): the library's rule on cells and width."""
-    cells = geom.nx * geom.ny * geom.nz
-    return cells >= 1.5e6 if geom.dtype == _native.FDTD_F64 else cells >= 4e6 and geom.nx >= 160
-
-
 def apply(sim, choice):
     """Set a choice on a NativeSim."""
     sim.set_option(_native.OPT_KERNEL, choice['kernel'])
