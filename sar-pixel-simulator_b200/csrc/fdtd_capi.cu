@@ -485,6 +485,28 @@ bool takes_pair(const fdtd_sim* s) {
          (s->esz == 8 ? cells >= kPairCellsDouble : cells >= kPairCellsFloat && s->g.nx >= kPairNxFloat);
 }
 
+// The fused step's tile and plan for the handle's settings: made before any
+// step, so that settings it does not take are refused on every path.
+int fused_ready(fdtd_sim* s) {
+  const fdtd_geometry& g = s->g;
+  if (!fused_supported_tile(s->tile_x, s->tile_y, (int)s->esz))
+    return fail(FDTD_ERR_INVALID, "unsupported fused tile %dx%d", s->tile_x, s->tile_y);
+  if (s->plan_ok && s->plan_tile_y == s->tile_y && s->plan_zchunk == s->zchunk && s->plan_slab == s->slab &&
+      s->plan_shell == s->shell)
+    return FDTD_OK;
+  s->plan_ok = 0;
+  s->plan = make_fused_plan(g.nx, g.ny, g.nz, g.npml, g.tfsf_z, s->tile_y, s->zchunk, s->slab,
+                            s->shell == FDTD_SHELL_MARCH);
+  if (s->plan.shell.dropped || s->plan.mshell.dropped)
+    return fail(FDTD_ERR_INVALID, "fused plan needs more than %d shell boxes", kMaxShellBoxes);
+  s->plan_tile_y = s->tile_y;
+  s->plan_zchunk = s->zchunk;
+  s->plan_slab = s->slab;
+  s->plan_shell = s->shell;
+  s->plan_ok = 1;
+  return FDTD_OK;
+}
+
 // Steps of each resident launch of a run of n: about a millisecond, because a
 // launch holds every SM and the work of other streams and handles waits for its
 // end (even: the launch then never updates H in place). A step takes about
@@ -499,6 +521,8 @@ unsigned long long wait_ns(const fdtd_sim* s) { return 1000ull * (unsigned long 
 
 template <class T>
 int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
+  if (s->kernel == FDTD_KERNEL_FUSED)
+    if (const int rc = fused_ready(s)) return rc;
   if (takes_resident<T>(s, n)) {
     if (const int rc = room_for_timing(s)) return rc;
     cudaEvent_t e0 = s->timing ? timing_event(s) : nullptr;
@@ -551,21 +575,6 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     s->path |= FDTD_PATH_SINGLE;
     if (s->kernel == FDTD_KERNEL_FUSED) {
       const int nxt = 1 - s->cur;
-      if (!fused_supported_tile(s->tile_x, s->tile_y, (int)sizeof(T)))
-        return fail(FDTD_ERR_INVALID, "unsupported fused tile %dx%d", s->tile_x, s->tile_y);
-      if (!s->plan_ok || s->plan_tile_y != s->tile_y || s->plan_zchunk != s->zchunk ||
-          s->plan_slab != s->slab || s->plan_shell != s->shell) {
-        const fdtd_geometry& g = s->g;
-        s->plan = make_fused_plan(g.nx, g.ny, g.nz, g.npml, g.tfsf_z, s->tile_y, s->zchunk, s->slab,
-                                  s->shell == FDTD_SHELL_MARCH);
-        s->plan_slab = s->slab;
-        s->plan_shell = s->shell;
-        if (s->plan.shell.dropped || s->plan.mshell.dropped)
-          return fail(FDTD_ERR_INVALID, "fused plan needs more than %d shell boxes", kMaxShellBoxes);
-        s->plan_tile_y = s->tile_y;
-        s->plan_zchunk = s->zchunk;
-        s->plan_ok = 1;
-      }
       // interior and shell H pass read the source set only; the shell E
       // pass reads the destination H that both of them wrote
       State<T> st = make_state<T>(s, s->cur, nxt);
@@ -2277,8 +2286,8 @@ int incident_run(fdtd_incident* b) {
   fdtd_sim* s = b->sim;
   const fdtd_geometry& g = s->g;
   b->ran = false;   // until this run is through
-  int rc = fdtd_reset(s);
-  if (rc) return rc;
+  int rc = s->kernel == FDTD_KERNEL_FUSED ? fused_ready(s) : FDTD_OK;
+  if (rc || (rc = fdtd_reset(s))) return rc;
   const size_t phb = (size_t)8 * s->ny_ph * s->nx_ph * s->esz;
   CK(cudaMemsetAsync(b->iph, 0, phb, s->stream));
   ShellBoxes whole;
