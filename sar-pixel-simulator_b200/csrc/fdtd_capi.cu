@@ -1485,7 +1485,8 @@ extern "C" int fdtd_near2far(const void* ex_u, const void* ey_u, const void* hx_
   const size_t pb = (size_t)nx_ph * ny_ph * (in_dtype == FDTD_F32 ? 8 : 16);
   const size_t ab = sizeof(double) * (size_t)(ntheta + nphi), ob = sizeof(double) * (size_t)8 * nphi * ntheta;
   const long long angles = (long long)nphi * ntheta;
-  const size_t sb = near2far_scratch(nx_ph, ny_ph, (int)std::min<long long>(angles, INT32_MAX));
+  int pass = (int)std::min<long long>(angles, kN2fPass);
+  size_t sb = near2far_scratch(nx_ph, ny_ph, pass);
   // one allocation: the planes as given, scratch, output, angles
   auto up = [](size_t n) { return (n + 255) / 256 * 256; };
   th.insert(th.end(), ph.begin(), ph.end());
@@ -1494,7 +1495,18 @@ extern "C" int fdtd_near2far(const void* ex_u, const void* ey_u, const void* hx_
   CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   int rc = FDTD_OK;
   do {
-    if (cudaMallocAsync((void**)&d, up(4 * pb) + up(sb) + up(ob) + up(ab), st) != cudaSuccess) {
+    // where memory is short, fewer directions at a time
+    cudaError_t e = cudaMallocAsync((void**)&d, up(4 * pb) + up(sb) + up(ob) + up(ab), st);
+    while (e != cudaSuccess && pass > 1) {
+      cudaGetLastError();
+      d = nullptr;
+      pass = std::max(pass / 8, 1);
+      sb = near2far_scratch(nx_ph, ny_ph, pass);
+      e = cudaMallocAsync((void**)&d, up(4 * pb) + up(sb) + up(ob) + up(ab), st);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      d = nullptr;
       rc = fail(FDTD_ERR_NOMEM, "near2far device allocation failed");
       break;
     }
@@ -1505,7 +1517,7 @@ extern "C" int fdtd_near2far(const void* ex_u, const void* ey_u, const void* hx_
     const void* planes[4] = {ex_u, ey_u, hx_u, hy_u};
     for (int c = 0; c < 4; ++c) cudaMemcpyAsync(d + c * pb, planes[c], pb, cudaMemcpyHostToDevice, st);
     if (near2far_run(d, in_dtype == FDTD_F32, nx_ph, ny_ph, dx, z_val, k, dth, ntheta, dth + ntheta, nphi, r, scratch,
-                     dout, st)) {
+                     pass, dout, st)) {
       rc = fail(FDTD_ERR_CUDA, "near2far launch failed: %s", cudaGetErrorString(cudaGetLastError()));
       break;
     }

@@ -26,7 +26,6 @@ namespace fdtd {
 namespace {
 
 constexpr int kN2fThreads = 256;
-constexpr int kN2fPass = 1024;   // directions of one pass (bounds the scratch)
 
 __device__ __forceinline__ double simpson_w(int i, int n) {
   if (i == 0 || i == n - 1) return 1.0;
@@ -199,17 +198,16 @@ k_n2f_finish(N2fAngles an, const double2* __restrict__ rows, const double2* __re
 
 }  // namespace
 
-size_t near2far_scratch(int nx, int ny, int angles) {
-  const size_t n = (size_t)(angles < kN2fPass ? angles : kN2fPass);
-  return n * ((size_t)nx + 5 * (size_t)ny) * sizeof(double2);
+size_t near2far_scratch(int nx, int ny, int pass) {
+  return (size_t)pass * ((size_t)nx + 5 * (size_t)ny) * sizeof(double2);
 }
 
 int near2far_run(const void* planes, bool single, int nx, int ny, double dx, double z_val, double k,
-                 const double* thetas, int ntheta, const double* phis, int nphi, double r, void* scratch, double* out,
-                 cudaStream_t st) {
+                 const double* thetas, int ntheta, const double* phis, int nphi, double r, void* scratch, int pass,
+                 double* out, cudaStream_t st) {
   const long long total = (long long)nphi * ntheta;
-  for (long long first = 0; first < total; first += kN2fPass) {
-    const int n = (int)(total - first < kN2fPass ? total - first : kN2fPass);
+  for (long long first = 0; first < total; first += pass) {
+    const int n = (int)(total - first < pass ? total - first : pass);
     const N2fAngles an{thetas, phis, ntheta, (int)first, n};
     double2* const fx = static_cast<double2*>(scratch);
     double2* const fy = fx + (size_t)n * nx;
