@@ -25,6 +25,7 @@ import numpy as np
 
 from . import _native
 from .absorbers import packed_profiles
+from .materials import MaterialModel, compute_material_arrays
 from .parameters import ParameterCollection
 
 ETA0 = 376.730313668
@@ -141,7 +142,14 @@ class BackscatterGradient:
         shape = (g.size_z_material, g.size_y, g.size_x)
         if eps_r.shape != shape:
             raise ValueError(f'material block must have shape {shape}, got {eps_r.shape}')
-        self.sim.set_materials_eps_sigma(eps_r, sigma)
+        try:
+            self.sim.set_materials_eps_sigma(eps_r, sigma)
+        except _native.FdtdError as e:
+            if e.code != _native.FDTD_ERR_NOMEM:
+                raise
+            # no room for the two staging volumes: made on the host, which
+            # needs none
+            self.sim.set_materials(*compute_material_arrays(self.params, MaterialModel(eps_r, sigma, g.cell_size)))
 
     def _upper_phasors(self):
         return np.stack([self.sim.get_phasor(k).astype(np.complex128) for k in (4, 5, 6, 7)])
