@@ -133,6 +133,7 @@ struct fdtd_sim {
   int wait_us = 2000000;                 // FDTD_OPT_WAIT_LIMIT_US
   bool side_by_side = false;             // running among a batch's streams
   int pair_state = 0;
+  int pair_pays = 0;                     // FDTD_MULTI_AUTO's rule: 0 not looked at, 1 yes, -1 no
   PairPlan pair;
   PairMapSet pmaps[2];
   void* pair_mid = nullptr;              // the planes of a PairMid
@@ -449,8 +450,6 @@ int enqueue_pair(fdtd_sim* s, int k, int ph_g0, int ph_ng, cudaEvent_t after_ste
   return FDTD_OK;
 }
 
-// ph_g0, ph_ng: the phasor plane groups each step accumulates (all six by
-// default; none with ph_ng = 0; the gradient's forward only the upper plane)
 // The path of a run of n steps. FDTD_MULTI_AUTO takes the fastest of the
 // three on the B200 (us per step; single, resident, pair):
 //   float  0.44 M cells  39  17  40      double  0.44 M   62   27   60
@@ -459,12 +458,53 @@ int enqueue_pair(fdtd_sim* s, int k, int ph_g0, int ph_ng, cudaEvent_t after_ste
 //          4.32 M       104 117  91              4.32 M  257  226  174
 //          14.7 M       230 376 186              14.7 M  635  769  328
 // The resident step wins while the fields (E, two sets of H, Ca, Cb) stay in
-// the 126 MB L2. The pair step wins once the plain box outweighs its ends:
-// in float also only on wide grids (91 x 267 x 133 cells: 92 single, 104
-// pair; 301 x 121 x 121: 116 and 135; 61 x 401 x 201: 125 and 111).
-constexpr long long kResidentBytes = 128LL << 20;
+// the 126 MB L2; in float, above 100 MB only where little of the grid is the
+// single step's interior box (45 x 383 x 74: 54 and 40; 52 x 85 x 670: 69 and
+// 88). The pair step wins once the plain box outweighs its ends: in float
+// also only on wide grids (91 x 267 x 133 cells: 92 single, 104 pair; 301 x
+// 121 x 121: 116 and 135; 61 x 401 x 201: 125 and 111), and not on thin ones
+// (800 x 34 x 200: 148 and 186; 26 x 939 x 177: 116 and 130), which the two
+// estimates tell apart. Of 348 float grids of 4 to 60 M cells drawn at random
+// pairs were slower on 67, by up to 24 %; on the 261 that the rule leaves
+// them they are slower on 5 by more than 2 %, by 6 % at most, and on the rest
+// they were 2 % slower on average. Of 171 for the resident step: 15 slower, by
+// up to 28 %; 3 of the 147 left, by 7 % at most. In double none of 185 was.
+constexpr long long kResidentBytes = 128LL << 20, kResidentBytesInterior = 100LL << 20;
+constexpr double kResidentInterior = 0.32;
 constexpr long long kPairCellsFloat = 4000000, kPairCellsDouble = 1500000;
 constexpr int kPairNxFloat = 160;
+constexpr double kPairMargin = 0.98;
+
+// Sides of the single step's interior box (make_fused_plan, without the planes
+// at the injection).
+void interior_box(const fdtd_geometry& g, double (&n)[3]) {
+  const int m = g.npml;
+  n[0] = std::max(0, (g.nx - m) / 4 * 4 - (m + 31) / 32 * 32);
+  n[1] = std::max(0, g.ny - 2 * m);
+  n[2] = std::max(0, g.nz - 2 * m);
+  if (n[0] * n[1] * n[2] == 0) n[0] = 0;
+}
+
+// Estimate of a single float step's time in us: its interior, the x, y and z
+// strips of its shell and the phasor planes, in cells (least squares over 378
+// grids of 3 to 60 M cells, 4 % rms).
+double single_us(const fdtd_geometry& g) {
+  double n[3];
+  interior_box(g, n);
+  const double nx = g.nx, ny = g.ny, nz = g.nz;
+  return 19.4 + 1e-6 * (9.0 * n[0] * n[1] * n[2] + 41 * nz * ny * (nx - n[0]) + 17.7 * nz * (ny - n[1]) * n[0] +
+                        14.2 * (nz - n[2]) * n[1] * n[0] + 76 * (ny * nx + nz * ny + nz * nx));
+}
+
+// Whether fields of these sizes run faster resident than in single steps.
+bool resident_pays(const fdtd_sim* s) {
+  const long long bytes = s->vol * 11 * (long long)s->esz;
+  if (bytes > kResidentBytes) return false;
+  if (s->esz == 8 || bytes <= kResidentBytesInterior) return true;
+  double n[3];
+  interior_box(s->g, n);
+  return n[0] * n[1] * n[2] < kResidentInterior * (double)s->g.nx * s->g.ny * s->g.nz;
+}
 
 template <class T>
 bool takes_resident(const fdtd_sim* s, int n) {
@@ -474,15 +514,22 @@ bool takes_resident(const fdtd_sim* s, int n) {
   // against 452)
   if (s->side_by_side) return false;
   if (s->multi == FDTD_MULTI_RESIDENT) return true;
-  return s->multi == FDTD_MULTI_AUTO && s->vol * 11 * (long long)sizeof(T) <= kResidentBytes;
+  return s->multi == FDTD_MULTI_AUTO && resident_pays(s);
 }
 
-bool takes_pair(const fdtd_sim* s) {
+bool takes_pair(fdtd_sim* s) {
   if (s->kernel != FDTD_KERNEL_FUSED || s->check_every > 0) return false;
   if (s->multi == FDTD_MULTI_PAIR) return true;
-  const long long cells = (long long)s->g.nx * s->g.ny * s->g.nz;
-  return s->multi == FDTD_MULTI_AUTO &&
-         (s->esz == 8 ? cells >= kPairCellsDouble : cells >= kPairCellsFloat && s->g.nx >= kPairNxFloat);
+  if (s->multi != FDTD_MULTI_AUTO) return false;
+  const fdtd_geometry& g = s->g;
+  const long long cells = (long long)g.nx * g.ny * g.nz;
+  if (s->esz == 8) return cells >= kPairCellsDouble;
+  if (cells < kPairCellsFloat || g.nx < kPairNxFloat) return false;
+  if (!s->pair_pays) {
+    const PairPlan p = make_pair_plan(g.nx, g.ny, g.nz, g.npml, 4);
+    s->pair_pays = p.ok && p.us < kPairMargin * single_us(g) ? 1 : -1;
+  }
+  return s->pair_pays > 0;
 }
 
 // The fused step's tile and plan for the handle's settings: made before any
@@ -519,6 +566,8 @@ int resident_launch_steps(const fdtd_sim* s, int n) {
 
 unsigned long long wait_ns(const fdtd_sim* s) { return 1000ull * (unsigned long long)s->wait_us; }
 
+// ph_g0, ph_ng: the phasor plane groups each step accumulates (all six by
+// default; none with ph_ng = 0; the gradient's forward only the upper plane)
 template <class T>
 int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
   if (s->kernel == FDTD_KERNEL_FUSED)
@@ -2323,7 +2372,9 @@ int incident_run(fdtd_incident* b) {
   launch_shell_pass<T>(st, zero_t, 0, whole, false, s->stream);
   source(0, 0);
   bool done = false;
-  if (takes_resident<T>(s, g.nt)) {
+  // by bytes alone: its single steps take two launches more each
+  const bool small = s->multi == FDTD_MULTI_AUTO && s->vol * 11 * (long long)sizeof(T) <= kResidentBytes;
+  if (takes_resident<T>(s, g.nt) || (small && s->kernel == FDTD_KERNEL_FUSED && g.nt >= 2)) {
     // resident launches, the source and the read-out with the steps
     const IncidentBeam<T> beam = {r, (const T*)b->exc[0], (const T*)b->exc[1], b->feed_in, b->nt_pulse};
     T* const other[3] = {(T*)s->fld[1][3], (T*)s->fld[1][4], (T*)s->fld[1][5]};

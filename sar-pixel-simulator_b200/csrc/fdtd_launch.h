@@ -231,7 +231,8 @@ struct PairRegions {
   PairRegion r[2];
 };
 struct PairPlan {
-  int ok;   // the grid has a plain box worth marching
+  int ok;      // the grid has a plain box worth marching
+  double us;   // estimate of a step's time, float
   PairRegions plain, zface, yend, xend;
 };
 enum PairKind { kPairPlain = 0, kPairZ, kPairY, kPairX };
