@@ -1534,8 +1534,8 @@ extern "C" int fdtd_near2far(const void* ex_u, const void* ey_u, const void* hx_
   const size_t pb = (size_t)nx_ph * ny_ph * (in_dtype == FDTD_F32 ? 8 : 16);
   const size_t ab = sizeof(double) * (size_t)(ntheta + nphi), ob = sizeof(double) * (size_t)8 * nphi * ntheta;
   const long long angles = (long long)nphi * ntheta;
-  int pass = (int)std::min<long long>(angles, kN2fPass);
-  size_t sb = near2far_scratch(nx_ph, ny_ph, pass);
+  int pass = near2far_pass(nx_ph, ny_ph, angles);
+  size_t sb = near2far_scratch(nx_ph, ny_ph, angles, pass);
   // one allocation: the planes as given, scratch, output, angles
   auto up = [](size_t n) { return (n + 255) / 256 * 256; };
   th.insert(th.end(), ph.begin(), ph.end());
@@ -1550,7 +1550,7 @@ extern "C" int fdtd_near2far(const void* ex_u, const void* ey_u, const void* hx_
       cudaGetLastError();
       d = nullptr;
       pass = std::max(pass / 8, 1);
-      sb = near2far_scratch(nx_ph, ny_ph, pass);
+      sb = near2far_scratch(nx_ph, ny_ph, angles, pass);
       e = cudaMallocAsync((void**)&d, up(4 * pb) + up(sb) + up(ob) + up(ab), st);
     }
     if (e != cudaSuccess) {

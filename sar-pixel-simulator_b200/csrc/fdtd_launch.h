@@ -363,10 +363,10 @@ int report_error(int code, const char* msg);
 // Near-to-far transform (near2far.cu) of the planes ex, ey, hx, hy as given
 // (complex64 with `single`, else complex128; device, one after another) into
 // out (4 x (nphi, ntheta) complex128, device); angles in radians (device).
-// The directions go in passes of `pass`; scratch: near2far_scratch bytes.
-// Returns 0 or 1 (CUDA error).
-constexpr int kN2fPass = 1024;   // bounds the scratch (73 MB for a 741 x 741 plane)
-size_t near2far_scratch(int nx, int ny, int pass);
+// The directions go in passes of `pass` (near2far_pass, or fewer); scratch:
+// near2far_scratch bytes. Returns 0 or 1 (CUDA error).
+int near2far_pass(int nx, int ny, long long angles);
+size_t near2far_scratch(int nx, int ny, long long angles, int pass);
 int near2far_run(const void* planes, bool single, int nx, int ny, double dx, double z_val, double k,
                  const double* thetas, int ntheta, const double* phis, int nphi, double r, void* scratch, int pass,
                  double* out, cudaStream_t st);

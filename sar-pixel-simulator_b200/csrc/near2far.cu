@@ -86,10 +86,12 @@ __global__ void __launch_bounds__(kN2fThreads) k_n2f_factors(N2fAngles an, int n
 constexpr int kN2fTile = 64, kN2fK = 16;   // 4 x 4 complex sums per thread of 256
 
 // R[a][y * 4 + c] = sum_x fx[a][x] P_c[y][x] for a tile of 64 directions by
-// 64 columns; planes: P_0 .. P_3, (ny, nx) each, one after another.
+// 64 columns; planes: P_0 .. P_3, (ny, nx) each, one after another. Where
+// there are few tiles of long rows, part z of `parts` sums every cell of its
+// share of the rows, into its own R.
 template <class C>
 __global__ void __launch_bounds__(kN2fThreads)
-k_n2f_rows(const C* __restrict__ planes, const double2* __restrict__ fx, int count, int nx, int ny,
+k_n2f_rows(const C* __restrict__ planes, const double2* __restrict__ fx, int count, int nx, int ny, int part_cells,
            double2* __restrict__ out) {
   __shared__ double2 sa[kN2fK][kN2fTile + 1], sp[kN2fK][kN2fTile + 1];
   const int a0 = blockIdx.x * kN2fTile, j0 = blockIdx.y * kN2fTile, cols = 4 * ny;
@@ -99,15 +101,17 @@ k_n2f_rows(const C* __restrict__ planes, const double2* __restrict__ fx, int cou
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0.0, 0.0);
-  for (int x0 = 0; x0 < nx; x0 += kN2fK) {
+  const int x_end = min(nx, (int)(blockIdx.z + 1) * part_cells);
+  out += (size_t)blockIdx.z * count * cols;
+  for (int x0 = blockIdx.z * part_cells; x0 < x_end; x0 += kN2fK) {
     // 16 threads read 16 consecutive x of a direction or plane row
     const int x = x0 + tx;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int a = a0 + ty + 16 * i, j = j0 + ty + 16 * i;
-      sa[tx][ty + 16 * i] = x < nx && a < count ? fx[(size_t)a * nx + x] : make_double2(0.0, 0.0);
+      sa[tx][ty + 16 * i] = x < x_end && a < count ? fx[(size_t)a * nx + x] : make_double2(0.0, 0.0);
       double2 v = make_double2(0.0, 0.0);
-      if (x < nx && j < cols) {
+      if (x < x_end && j < cols) {
         const C q = planes[((size_t)(j & 3) * ny + (j >> 2)) * nx + x];
         v = make_double2((double)q.x, (double)q.y);
       }
@@ -141,11 +145,11 @@ k_n2f_rows(const C* __restrict__ planes, const double2* __restrict__ fx, int cou
     }
 }
 
-// One block per direction: the sums of R over y against fy, then the
-// potentials and the far field.
+// One block per direction: the sums of R over y against fy (and over its
+// parts), then the potentials and the far field.
 __global__ void __launch_bounds__(kN2fThreads)
-k_n2f_finish(N2fAngles an, const double2* __restrict__ rows, const double2* __restrict__ fy, int ny, double dx,
-             double k, double r, long long plane, double2* __restrict__ out) {
+k_n2f_finish(N2fAngles an, const double2* __restrict__ rows, int parts, const double2* __restrict__ fy, int ny,
+             double dx, double k, double r, long long plane, double2* __restrict__ out) {
   const int a = blockIdx.x;
   // sums of ex, ey, hx, hy (re, im)
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -153,7 +157,11 @@ k_n2f_finish(N2fAngles an, const double2* __restrict__ rows, const double2* __re
     const double2 f = fy[(size_t)a * ny + y];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const double2 v = rows[((size_t)a * ny + y) * 4 + c];
+      double2 v = rows[((size_t)a * ny + y) * 4 + c];
+      for (int p = 1; p < parts; ++p) {
+        const double2 w = rows[(((size_t)p * an.count + a) * ny + y) * 4 + c];
+        v = make_double2(v.x + w.x, v.y + w.y);
+      }
       acc[2 * c] += f.x * v.x - f.y * v.y;
       acc[2 * c + 1] += f.x * v.y + f.y * v.x;
     }
@@ -198,8 +206,35 @@ k_n2f_finish(N2fAngles an, const double2* __restrict__ rows, const double2* __re
 
 }  // namespace
 
-size_t near2far_scratch(int nx, int ny, int pass) {
-  return (size_t)pass * ((size_t)nx + 5 * (size_t)ny) * sizeof(double2);
+namespace {
+
+// Parts of the rows' sums: one, unless a plane of rows of 512 cells or more
+// leaves 16 tiles or fewer, whose sums would run one after another on as many
+// SMs (4 directions of 3 x 20001 cells: 6.3 ms in one part, 1.0 in 148). By the
+// call's directions, not the pass's: a sum does not depend on how much memory
+// there is.
+int row_parts(int nx, int ny, long long angles) {
+  const long long tiles = ((angles + kN2fTile - 1) / kN2fTile) * ((4LL * ny + kN2fTile - 1) / kN2fTile);
+  return nx >= 512 && tiles <= 16 ? (int)(148 / tiles < nx / 64 ? 148 / tiles : nx / 64) : 1;
+}
+
+size_t direction_bytes(int nx, int ny, int parts) {
+  return ((size_t)nx + (size_t)ny * (1 + 4 * (size_t)parts)) * sizeof(double2);
+}
+
+}  // namespace
+
+// A pass of 1024 directions, or as many as 32 MB hold where planes are small
+// (a pass is three launches; 16384 directions of 19 x 19 cells: 1.3 ms in
+// passes of 1024, 1.0 so).
+int near2far_pass(int nx, int ny, long long angles) {
+  const long long most = (32LL << 20) / (long long)direction_bytes(nx, ny, 1);
+  const long long n = most < 1024 ? 1024 : most > 65535 ? 65535 : most;
+  return (int)(angles < n ? angles : n);
+}
+
+size_t near2far_scratch(int nx, int ny, long long angles, int pass) {
+  return (size_t)pass * direction_bytes(nx, ny, row_parts(nx, ny, angles));
 }
 
 int near2far_run(const void* planes, bool single, int nx, int ny, double dx, double z_val, double k,
@@ -214,10 +249,14 @@ int near2far_run(const void* planes, bool single, int nx, int ny, double dx, dou
     double2* const rows = fy + (size_t)n * ny;
     k_n2f_factors<<<dim3((nx + ny + kN2fThreads - 1) / kN2fThreads, n), kN2fThreads, 0, st>>>(an, nx, ny, dx, z_val, k,
                                                                                               fx, fy);
-    const dim3 grd((n + kN2fTile - 1) / kN2fTile, (4 * ny + kN2fTile - 1) / kN2fTile);
-    if (single) k_n2f_rows<float2><<<grd, kN2fThreads, 0, st>>>(static_cast<const float2*>(planes), fx, n, nx, ny, rows);
-    else k_n2f_rows<double2><<<grd, kN2fThreads, 0, st>>>(static_cast<const double2*>(planes), fx, n, nx, ny, rows);
-    k_n2f_finish<<<n, kN2fThreads, 0, st>>>(an, rows, fy, ny, dx, k, r, total, reinterpret_cast<double2*>(out));
+    const int parts = row_parts(nx, ny, total), cells = ((nx + parts - 1) / parts + kN2fK - 1) / kN2fK * kN2fK;
+    const dim3 grd((n + kN2fTile - 1) / kN2fTile, (4 * ny + kN2fTile - 1) / kN2fTile, parts);
+    if (single)
+      k_n2f_rows<float2><<<grd, kN2fThreads, 0, st>>>(static_cast<const float2*>(planes), fx, n, nx, ny, cells, rows);
+    else
+      k_n2f_rows<double2><<<grd, kN2fThreads, 0, st>>>(static_cast<const double2*>(planes), fx, n, nx, ny, cells, rows);
+    k_n2f_finish<<<n, kN2fThreads, 0, st>>>(an, rows, parts, fy, ny, dx, k, r, total,
+                                            reinterpret_cast<double2*>(out));
   }
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
