@@ -2372,9 +2372,7 @@ int incident_run(fdtd_incident* b) {
   launch_shell_pass<T>(st, zero_t, 0, whole, false, s->stream);
   source(0, 0);
   bool done = false;
-  // by bytes alone: its single steps take two launches more each
-  const bool small = s->multi == FDTD_MULTI_AUTO && s->vol * 11 * (long long)sizeof(T) <= kResidentBytes;
-  if (takes_resident<T>(s, g.nt) || (small && s->kernel == FDTD_KERNEL_FUSED && g.nt >= 2)) {
+  if (takes_resident<T>(s, g.nt)) {
     // resident launches, the source and the read-out with the steps
     const IncidentBeam<T> beam = {r, (const T*)b->exc[0], (const T*)b->exc[1], b->feed_in, b->nt_pulse};
     T* const other[3] = {(T*)s->fld[1][3], (T*)s->fld[1][4], (T*)s->fld[1][5]};

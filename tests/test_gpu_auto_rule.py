@@ -6,7 +6,9 @@ import numpy as np
 import pytest
 
 from fdtdsarsim_b200 import _native
-from helpers import make_params, native_for
+from fdtdsarsim_b200.absorbers import packed_profiles
+from fdtdsarsim_b200.gpu.main_sim import native_geometry
+from helpers import bits_equal, make_params, native_for
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +34,23 @@ def test_auto_takes_the_faster_path(nz, ny, nx, dtype, want):
     taken = sim.get_option(_native.OPT_STEP_PATH)
     sim.close()
     assert taken == want
+
+
+@pytest.mark.parametrize('nz,ny,nx', [(52, 85, 670), (45, 383, 74)])
+def test_incident_run_by_the_same_rule_equals_split(nz, ny, nx):
+    """Single steps on the first grid (resident 5.4 ms per 60 steps, single
+    4.7), resident ones on the second."""
+    nt = 8
+    pc = make_params(nx, ny, nz, nz // 2, nt, 0, cell_wl=0.05)
+    src = np.random.default_rng(nx).standard_normal((2, nt, ny, nx)).astype('float32')
+    out = []
+    for opts in ({}, {_native.OPT_KERNEL: _native.FDTD_KERNEL_SPLIT}):
+        inc = _native.NativeIncident(native_geometry(pc), nt, 0)
+        inc.set_absorbers(packed_profiles(pc))
+        for k, v in opts.items():
+            inc.set_option(k, v)
+        inc.set_excitation(src[0], src[1])
+        inc.run()
+        out.append({**inc.get_planes(), **inc.get_phasors()})
+        inc.close()
+    assert all(bits_equal(out[0][k], out[1][k]) and np.any(out[1][k]) for k in out[1])
