@@ -82,7 +82,9 @@ extern "C" {
 #define FDTD_OPT_MULTISTEP    13 /* FDTD_MULTI_*: FDTD_KERNEL_FUSED may
                                     advance several steps per launch, with the
                                     same results bit for bit (default 0). Not
-                                    used while FDTD_OPT_CHECK_EVERY is on */
+                                    used while FDTD_OPT_CHECK_EVERY is on, nor
+                                    in float on cells of 2 m or more (but
+                                    powers of two) */
 #define FDTD_OPT_WAIT_LIMIT_US 14 /* longest wait, in us, of a resident launch's
                                     blocks for one another (default 2000000, at
                                     most 10 s). When it runs out the launch ends,

@@ -506,9 +506,16 @@ bool resident_pays(const fdtd_sim* s) {
   return n[0] * n[1] * n[2] < kResidentInterior * (double)s->g.nx * s->g.ny * s->g.nz;
 }
 
+// Several steps per launch: for the fused step, with no look at the fields after
+// every step, and a cell size that div_off_boundary takes.
+bool takes_several(const fdtd_sim* s) {
+  return s->kernel == FDTD_KERNEL_FUSED && s->check_every == 0 &&
+         (s->esz == 8 || !has_boundary_quotients((float)s->g.cell_size));
+}
+
 template <class T>
 bool takes_resident(const fdtd_sim* s, int n) {
-  if (s->kernel != FDTD_KERNEL_FUSED || s->check_every > 0 || n < 2) return false;
+  if (!takes_several(s) || n < 2) return false;
   // members that run side by side: a launch that takes every SM would run
   // them one after another (10 members of 0.6 to 4 M cells: 507 us per step
   // against 452)
@@ -518,7 +525,7 @@ bool takes_resident(const fdtd_sim* s, int n) {
 }
 
 bool takes_pair(fdtd_sim* s) {
-  if (s->kernel != FDTD_KERNEL_FUSED || s->check_every > 0) return false;
+  if (!takes_several(s)) return false;
   if (s->multi == FDTD_MULTI_PAIR) return true;
   if (s->multi != FDTD_MULTI_AUTO) return false;
   const fdtd_geometry& g = s->g;

@@ -189,6 +189,18 @@ __device__ __forceinline__ float div_const(float u, float, double r) {
   const double q = __dmul_rn((double)u, r);
   return __double2float_rn(__hiloint2double(__double2hiint(q), __double2loint(q) & ~3));
 }
+// The same for a d with which no quotient lies on a boundary, or a power of two
+// (whose products are exact): the two bits can stay. The resident and the pair
+// step divide so, and leave other cell sizes to the single step (a pair of
+// 101 x 381 x 381 cells: 358 us so, 363 with the bits cleared; 203 x 761 x 761:
+// 1870 and 1881).
+__device__ __forceinline__ float div_off_boundary(float u, float, double r) {
+  return __double2float_rn(__dmul_rn((double)u, r));
+}
+inline bool has_boundary_quotients(float d) {
+  int e;
+  return d >= 2.0f && std::frexp(d, &e) != 0.5f;
+}
 inline double div_reciprocal(float d) {
   const double r = 1.0 / (double)d;
   return std::fma(r, (double)d, -1.0) < 0.0 ? std::nextafter(r, INFINITY) : r;
@@ -212,6 +224,9 @@ __device__ __forceinline__ double div_const(double u, double d, double r) {
   }
   return a == 0.0 ? u : __ddiv_rn(u, d);   // zeros keep their sign; tiny, huge, NaN: IEEE
 }
+
+__device__ __forceinline__ double div_off_boundary(double u, double d, double r) { return div_const(u, d, r); }
+inline bool has_boundary_quotients(double) { return false; }
 
 template <class T>
 __device__ __forceinline__ T div_dx(const State<T>& s, T u) { return div_const(u, s.dx, s.rdx64); }

@@ -22,14 +22,16 @@ __device__ __forceinline__ bool same_bits_d(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b) || (a != a && b != b);
 }
 
-__global__ void k_check_div_f(float d, double r, unsigned long long* bad) {
+// off: the form without the cleared bits is to be exact too.
+__global__ void k_check_div_f(float d, double r, bool off, unsigned long long* bad) {
   unsigned long long local = 0;
   const unsigned long long n = 1ULL << 32;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += stride) {
     const float u = __uint_as_float((unsigned)k);
-    if (!same_bits_f(div_const(u, d, r), __fdiv_rn(u, d))) ++local;
+    const float q = __fdiv_rn(u, d);
+    if (!same_bits_f(div_const(u, d, r), q) || (off && !same_bits_f(div_off_boundary(u, d, r), q))) ++local;
   }
   if (local) atomicAdd(bad, local);
 }
@@ -83,7 +85,7 @@ extern "C" int fdtd_check_cell_division(int dtype, double cell_size, int device,
     const float d = (float)cell_size;
     const double r = div_reciprocal(d);
     n = 1ULL << 32;
-    k_check_div_f<<<148 * 16, 256>>>(d, r, bad);
+    k_check_div_f<<<148 * 16, 256>>>(d, r, !has_boundary_quotients(d), bad);
   } else {
     const double r = div_reciprocal(cell_size);
     n = 1ULL << 30;

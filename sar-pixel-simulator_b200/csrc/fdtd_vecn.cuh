@@ -113,8 +113,8 @@ __device__ __forceinline__ void psi_pair(const State<T>& s, T mz, const T (&b)[V
   vmul(q1, c, d1, mz);
 #pragma unroll
   for (int j = 0; j < V; ++j) {
-    q0[j] = div_dx(s, q0[j]);
-    q1[j] = div_dx(s, q1[j]);
+    q0[j] = div_off_boundary(q0[j], s.dx, s.rdx64);
+    q1[j] = div_off_boundary(q1[j], s.dx, s.rdx64);
   }
   vmul(p0, b, p0, mz);
   vmul(p1, b, p1, mz);
