@@ -263,8 +263,8 @@ def job_rate(units, steps, ms, world):
 
 def run_launches(choice, steps, path):
     """Kernel launches of one run of `steps` steps that took `path`
-    (FDTD_OPT_STEP_PATH): resident steps, one launch (at least: one per
-    millisecond) and the counter's; a pair of steps, one march of each of the
+    (FDTD_OPT_STEP_PATH): resident steps, one launch (at least: one per two
+    milliseconds) and the counter's; a pair of steps, one march of each of the
     four regions and the phasors; otherwise step_launches a step, and the
     counter's."""
     from fdtdsarsim_b200 import _native

@@ -106,7 +106,7 @@ extern "C" {
 #define FDTD_MULTI_AUTO     1 /* by the grid's size: resident, pair or single */
 #define FDTD_MULTI_RESIDENT 2 /* many steps per cooperative launch (not among
                                  a batch's streams). A launch holds every SM
-                                 for about a millisecond; work of other
+                                 for about two milliseconds; work of other
                                  streams and handles runs between launches */
 #define FDTD_MULTI_PAIR     3 /* two steps per pass over the fields; holds a
                                  few planes more, allocated on the first run

@@ -561,13 +561,13 @@ int fused_ready(fdtd_sim* s) {
   return FDTD_OK;
 }
 
-// Steps of each resident launch of a run of n: about a millisecond, because a
+// Steps of each resident launch of a run of n: about two milliseconds, because a
 // launch holds every SM and the work of other streams and handles waits for its
 // end (even: the launch then never updates H in place). A step takes about
 // 7 us and 1 us per 150 KB of one field (the sizes above).
 int resident_launch_steps(const fdtd_sim* s, int n) {
   const double us = 7.0 + (double)s->vol * s->esz / 150e3;
-  const int most = std::max(2, (int)(1000.0 / us)), launches = (n + most - 1) / most;
+  const int most = std::max(2, (int)(2000.0 / us)), launches = (n + most - 1) / most;
   return ((n + launches - 1) / launches + 1) & ~1;
 }
 

@@ -11,9 +11,11 @@
 // sets, so that the phasors of the finished step can read its H beside the
 // H pass that follows. The last of an odd number of steps updates H in place
 // (after its predecessor's phasors), so that a launch ends on the set it began
-// with. A launch is of about a millisecond (resident_launch_steps,
-// fdtd_capi.cu), because it holds every SM: a run of one launch instead of
-// one per millisecond is 0.4 % to 0.9 % faster, but stops every other stream. The updates are the split passes' (fdtd_split.cuh), bit for bit.
+// with. A launch is of about two milliseconds (resident_launch_steps,
+// fdtd_capi.cu), because it holds every SM and stops every other stream; one
+// launch for the whole run is 0.2 % faster (one per millisecond 0.8 % slower).
+// The updates are those of fdtd_vecn.cuh, equal bit for bit to the split
+// passes'; the phasor cell is the split step's (fdtd_split.cuh).
 //
 // The barrier waits with a time limit, after which every block leaves and
 // the launch is reported as failed.

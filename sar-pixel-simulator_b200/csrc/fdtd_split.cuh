@@ -1,6 +1,6 @@
-// fdtd_split.cuh -- the split step's H and E updates of one vector and the
-// phasor update of one cell, shared by the split passes (fdtd_split.cu) and
-// the resident step (fdtd_resident.cu).
+// fdtd_split.cuh -- the split step's H and E updates of one vector, for the
+// split passes (fdtd_split.cu), and the phasor update of one cell, which the
+// resident step (fdtd_resident.cu) shares.
 #pragma once
 
 #include "fdtd_vec.cuh"

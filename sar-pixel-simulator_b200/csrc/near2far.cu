@@ -302,8 +302,9 @@ static __device__ __align__(256) unsigned char g_n2f_scratch[kN2fScratchBytes];
 std::mutex g_n2f_mutex;
 void* g_n2f_addr[64] = {};   // device address of g_n2f_scratch, per device
 
-// Same integration as k_near2far, reading the u-plane phasors as given
-// (complex64 or complex128), forming J = (-Hy, Hx), M = (Ey, -Ex) on the fly
+// One block per direction with a sine and cosine per cell (fdtd_near2far's
+// matrix product needs scratch beyond the static array), reading the u-plane
+// phasors as given (complex64 or complex128), forming J = (-Hy, Hx), M = (Ey, -Ex) on the fly
 // and converting the angles from degrees on the device.
 template <class C>
 __global__ void __launch_bounds__(kN2fThreads)

@@ -1,5 +1,5 @@
-"""A resident run leaves the device to others between its launches of about a
-millisecond: work of another stream, and another simulation, finish while a
+"""A resident run leaves the device to others between its launches of about two
+milliseconds: work of another stream, and another simulation, finish while a
 long run is still going."""
 import pytest
 
