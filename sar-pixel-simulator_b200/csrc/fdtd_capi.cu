@@ -76,11 +76,8 @@ struct fdtd_sim {
   long long ph_off[24];
   long long ph_elems = 0;
   double* phase = nullptr;
-  int* tdev = nullptr;                   // step counter; [2] stays 0; [4], [5] the resident step's barrier
-  // page-locked host word that a kernel sets when a wait inside it ran out:
-  // read after a synchronisation without a copy on the legacy default
-  // stream, which would wait for other streams
-  int* waited = nullptr;
+  int* tdev = nullptr;                   // step counter; [2] stays 0; [4], [5] the resident step's barrier;
+                                         // [6] set by a kernel when a wait inside it ran out
   int* flags = nullptr;                  // non-finite check: found, step
   int64_t t = 0;
   int cur = 0;
@@ -139,6 +136,9 @@ struct fdtd_sim {
   void* pair_mid = nullptr;              // the planes of a PairMid
   cudaStream_t side2 = nullptr;
   cudaEvent_t join2 = nullptr;
+  // kernels that wait were enqueued since the last look at their word, or lie in
+  // a caller's graph; one of them had its wait run out (until a reset)
+  bool wait_look = false, wait_captured = false, wait_failed = false;
   // captured step chunks (FDTD_OPT_GRAPH_CHUNK), one per starting field set,
   // with the settings they were captured under; absorber uploads bump the
   // epoch (the profiles are captured by value)
@@ -147,6 +147,7 @@ struct fdtd_sim {
   int gend[2] = {};                      // the current set after a replay
   int gpath[2] = {};                     // the paths it holds
   int path = 0;                          // FDTD_OPT_STEP_PATH: those of the last run
+  bool capturing = false;                // a chunk of the handle's own
   int graph_epoch = 0;
   // gradient (fdtd_grad_*): checkpoints of the forward solve, the segment
   // of recomputed states and the adjoint state; a state is the 6 fields
@@ -240,10 +241,18 @@ int take_bounds_violation() {
 }
 
 // A wait inside a kernel that ran out since the last reset: what the handle
-// holds is not valid, and every call that hands it out says so. After a
-// synchronisation of the handle's stream.
-int wait_error(const fdtd_sim* s) {
-  if (!*(const volatile int*)s->waited) return FDTD_OK;
+// holds is not valid, and every call that hands it out says so. The look is a
+// copy on the handle's stream (a page-locked word would need none, but made
+// fdtd_create 2.5 ms longer).
+int wait_error(fdtd_sim* s) {
+  if (!s->wait_failed && (s->wait_look || s->wait_captured)) {
+    int w = 0;
+    CK(cudaMemcpyAsync(&w, s->tdev + 6, sizeof(w), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    s->wait_look = false;
+    s->wait_failed = w != 0;
+  }
+  if (!s->wait_failed) return FDTD_OK;
   return fail(FDTD_ERR_CUDA, "a wait inside a step kernel ran out: the results are not valid (fdtd_reset)");
 }
 
@@ -377,6 +386,17 @@ int collect_timing(fdtd_sim* s) {
   return FDTD_OK;
 }
 
+// Kernels that wait follow on the handle's stream: to be looked at after the
+// run, and after every replay of a caller's graph that holds them (the
+// handle's own graphs are looked at where they are launched).
+void waits_enqueued(fdtd_sim* s) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (!s->capturing && cudaStreamIsCapturing(s->stream, &capture) == cudaSuccess &&
+      capture != cudaStreamCaptureStatusNone)
+    s->wait_captured = true;
+  s->wait_look = true;
+}
+
 // At most 4096 timed groups wait for collection.
 int room_for_timing(fdtd_sim* s) {
   return s->timing && s->ev_used + 3 > 3 * 4096 ? collect_timing(s) : FDTD_OK;
@@ -431,14 +451,15 @@ int enqueue_pair(fdtd_sim* s, int k, int ph_g0, int ph_ng, cudaEvent_t after_ste
     for (int t = 0; t < 2; ++t)
       for (int c = 0; c < 4; ++c, q += sizes[2]) mid.x[t][c] = q;
   }
+  waits_enqueued(s);
   CK(cudaEventRecord(s->fork, s->stream));
   CK(cudaStreamWaitEvent(s->side, s->fork, 0));
   CK(cudaStreamWaitEvent(s->side2, s->fork, 0));
   const PairMapSet& maps = s->pmaps[s->cur];
-  if (!launch_pair<T>(kPairX, st, s->pair, maps, mid, s->tdev, k, s->waited, s->side) ||
-      !launch_pair<T>(kPairY, st, s->pair, maps, mid, s->tdev, k, s->waited, s->side2) ||
-      !launch_pair<T>(kPairPlain, st, s->pair, maps, mid, s->tdev, k, s->waited, s->stream) ||
-      !launch_pair<T>(kPairZ, st, s->pair, maps, mid, s->tdev, k, s->waited, s->side2))
+  if (!launch_pair<T>(kPairX, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side) ||
+      !launch_pair<T>(kPairY, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side2) ||
+      !launch_pair<T>(kPairPlain, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->stream) ||
+      !launch_pair<T>(kPairZ, st, s->pair, maps, mid, s->tdev, k, s->tdev + 6, s->side2))
     return fail(FDTD_ERR_CUDA, "pair step launch: %s", cudaGetErrorString(cudaGetLastError()));
   CK(cudaEventRecord(s->join, s->side));
   CK(cudaEventRecord(s->join2, s->side2));
@@ -589,10 +610,11 @@ int enqueue_steps(fdtd_sim* s, int n, int ph_g0 = 0, int ph_ng = 6) {
     T* const other[3] = {(T*)s->fld[1 - s->cur][3], (T*)s->fld[1 - s->cur][4], (T*)s->fld[1 - s->cur][5]};
     const State<T> st = make_state<T>(s, s->cur, s->cur);
     const int each = resident_launch_steps(s, n);
+    waits_enqueued(s);
     int done = 0;
     while (done < n &&
            launch_resident<T>(st, other, s->tdev, done, std::min(each, n - done), ph_g0, ph_ng,
-                              (unsigned*)(s->tdev + 4), s->waited, wait_ns(s), s->stream))
+                              (unsigned*)(s->tdev + 4), s->tdev + 6, wait_ns(s), s->stream))
       done += std::min(each, n - done);
     mark(s, e1);
     mark(s, e2);
@@ -699,7 +721,9 @@ int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     const int before = s->path;
     s->path = 0;
+    s->capturing = true;
     const int rc = enqueue_steps<T>(s, chunk);
+    s->capturing = false;
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
     s->gpath[start] = s->path;
@@ -720,6 +744,7 @@ int enqueue_graph_chunk(fdtd_sim* s, int chunk) {
     memcpy(s->gsig[start], sig, sizeof(sig));
   }
   CK(cudaGraphLaunch(s->gexec[start], s->stream));
+  s->wait_look = s->wait_look || s->gpath[start] != FDTD_PATH_SINGLE;
   s->path |= s->gpath[start];
   s->cur = s->gend[start];
   return FDTD_OK;
@@ -881,11 +906,6 @@ int fdtd_create(const fdtd_geometry* geom, int device, fdtd_sim** out) {
   A((size_t)std::max(g.nt, 1) * 4 * sizeof(double), (void**)&s->phase);
   A(sizeof(int) * 8, (void**)&s->tdev);
   A(sizeof(int) * 2, (void**)&s->flags);
-  if (rc == FDTD_OK && cudaHostAlloc((void**)&s->waited, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
-    cudaGetLastError();
-    s->waited = nullptr;
-    rc = fail(FDTD_ERR_NOMEM, "no page-locked host memory");
-  }
   if (rc != FDTD_OK) {
     fdtd_destroy(s);
     return rc;
@@ -954,7 +974,6 @@ int fdtd_destroy(fdtd_sim* s) {
     if (s->stage[k]) cudaFreeHost(s->stage[k]);
   }
   if (s->copy) cudaStreamDestroy(s->copy);
-  if (s->waited) cudaFreeHost(s->waited);
   for (auto e : s->ev) cudaEventDestroy(e);
   for (int k = 0; k < 2; ++k)
     if (s->gexec[k]) cudaGraphExecDestroy(s->gexec[k]);
@@ -1266,7 +1285,7 @@ int fdtd_reset(fdtd_sim* s) {
   CK(cudaMemsetAsync(s->tdev, 0, sizeof(int) * 8, s->stream));
   CK(cudaMemsetAsync(s->flags, 0, sizeof(int) * 2, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  *s->waited = 0;
+  s->wait_look = s->wait_failed = false;
   s->t = 0;
   s->cur = 0;
   return FDTD_OK;
@@ -2384,9 +2403,10 @@ int incident_run(fdtd_incident* b) {
     const IncidentBeam<T> beam = {r, (const T*)b->exc[0], (const T*)b->exc[1], b->feed_in, b->nt_pulse};
     T* const other[3] = {(T*)s->fld[1][3], (T*)s->fld[1][4], (T*)s->fld[1][5]};
     const int each = resident_launch_steps(s, g.nt);
+    waits_enqueued(s);
     int t = 0;
     while (t < g.nt && launch_resident_beam<T>(st, other, beam, s->tdev, t, std::min(each, g.nt - t),
-                                               (unsigned*)(s->tdev + 4), s->waited, wait_ns(s), s->stream))
+                                               (unsigned*)(s->tdev + 4), s->tdev + 6, wait_ns(s), s->stream))
       t += std::min(each, g.nt - t);
     done = t == g.nt;
     if (t > 0 && !done)

@@ -201,7 +201,7 @@ struct ResidentArgs {
 // Enqueues nsteps steps from the step *tdev + toff (their phasors in plane
 // groups ph_g0 .. ph_g0 + ph_ng - 1 included); the run ends on the set it
 // began with. sync: two words of device memory, zero after a reset; *err
-// (host-mapped) is set when a barrier waited longer than wait_ns. False: not
+// (device) is set when a barrier waited longer than wait_ns. False: not
 // launched.
 template <class T>
 bool launch_resident(const State<T>& s, T* const other_h[3], const int* tdev, int toff, int nsteps, int ph_g0,
@@ -269,7 +269,7 @@ PairPlan make_pair_plan(int nx, int ny, int nz, int npml, int elem_bytes);
 template <class T>
 bool make_pair_maps(const State<T>& s, PairMapSet* out);
 // The march over the regions of one kind, source set -> destination set;
-// the four may run in any order or side by side. *err (host-mapped) is set when
+// the four may run in any order or side by side. *err (device) is set when
 // a plane's copy did not arrive in time.
 template <class T>
 bool launch_pair(PairKind kind, const State<T>& s, const PairPlan& p, const PairMapSet& maps, const PairMid<T>& mid,

@@ -97,3 +97,26 @@ def test_limits_out_of_range_are_refused(value):
     sim = native_for(make_params(27, 25, 23, 14, 4, 4))
     _fails(lambda: sim.set_option(_native.OPT_WAIT_LIMIT_US, value), _native.FDTD_ERR_INVALID, 'wait limit')
     sim.close()
+
+
+def test_a_callers_graph_reports_a_wait_of_any_replay():
+    import torch
+    pc = make_params(64, 57, 41, 20, 3 * NT, 3 * NT)
+    sim = _sim(pc, _native.MULTI_RESIDENT)
+    stream = torch.cuda.Stream()
+    sim.set_stream(stream.cuda_stream)
+    sim.set_option(_native.OPT_WAIT_LIMIT_US, 0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        sim.run(NT)
+    sim.synchronize()   # nothing has run
+    for _ in range(2):
+        with torch.cuda.stream(stream):
+            graph.replay()
+        _fails(sim.synchronize)
+        _fails(sim.get_phasors)
+        sim.reset()
+        sim.synchronize()
+    del graph
+    sim.set_stream(0)
+    sim.close()
