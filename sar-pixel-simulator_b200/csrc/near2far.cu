@@ -89,7 +89,7 @@ constexpr int kN2fTile = 64, kN2fK = 16;   // 4 x 4 complex sums per thread of 2
 // 64 columns; planes: P_0 .. P_3, (ny, nx) each, one after another. Where
 // there are few tiles of long rows, part z of `parts` sums every cell of its
 // share of the rows, into its own R.
-template <class C>
+template <class C, bool kParts>
 __global__ void __launch_bounds__(kN2fThreads)
 k_n2f_rows(const C* __restrict__ planes, const double2* __restrict__ fx, int count, int nx, int ny, int part_cells,
            double2* __restrict__ out) {
@@ -101,9 +101,9 @@ k_n2f_rows(const C* __restrict__ planes, const double2* __restrict__ fx, int cou
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0.0, 0.0);
-  const int x_end = min(nx, (int)(blockIdx.z + 1) * part_cells);
-  out += (size_t)blockIdx.z * count * cols;
-  for (int x0 = blockIdx.z * part_cells; x0 < x_end; x0 += kN2fK) {
+  const int x_end = kParts ? min(nx, (int)(blockIdx.z + 1) * part_cells) : nx;
+  if (kParts) out += (size_t)blockIdx.z * count * cols;
+  for (int x0 = kParts ? blockIdx.z * part_cells : 0; x0 < x_end; x0 += kN2fK) {
     // 16 threads read 16 consecutive x of a direction or plane row
     const int x = x0 + tx;
 #pragma unroll
@@ -147,6 +147,7 @@ k_n2f_rows(const C* __restrict__ planes, const double2* __restrict__ fx, int cou
 
 // One block per direction: the sums of R over y against fy (and over its
 // parts), then the potentials and the far field.
+template <bool kParts>
 __global__ void __launch_bounds__(kN2fThreads)
 k_n2f_finish(N2fAngles an, const double2* __restrict__ rows, int parts, const double2* __restrict__ fy, int ny,
              double dx, double k, double r, long long plane, double2* __restrict__ out) {
@@ -158,7 +159,7 @@ k_n2f_finish(N2fAngles an, const double2* __restrict__ rows, int parts, const do
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       double2 v = rows[((size_t)a * ny + y) * 4 + c];
-      for (int p = 1; p < parts; ++p) {
+      for (int p = 1; kParts && p < parts; ++p) {
         const double2 w = rows[(((size_t)p * an.count + a) * ny + y) * 4 + c];
         v = make_double2(v.x + w.x, v.y + w.y);
       }
@@ -251,12 +252,19 @@ int near2far_run(const void* planes, bool single, int nx, int ny, double dx, dou
                                                                                               fx, fy);
     const int parts = row_parts(nx, ny, total), cells = ((nx + parts - 1) / parts + kN2fK - 1) / kN2fK * kN2fK;
     const dim3 grd((n + kN2fTile - 1) / kN2fTile, (4 * ny + kN2fTile - 1) / kN2fTile, parts);
-    if (single)
-      k_n2f_rows<float2><<<grd, kN2fThreads, 0, st>>>(static_cast<const float2*>(planes), fx, n, nx, ny, cells, rows);
-    else
-      k_n2f_rows<double2><<<grd, kN2fThreads, 0, st>>>(static_cast<const double2*>(planes), fx, n, nx, ny, cells, rows);
-    k_n2f_finish<<<n, kN2fThreads, 0, st>>>(an, rows, parts, fy, ny, dx, k, r, total,
-                                            reinterpret_cast<double2*>(out));
+    double2* const o = reinterpret_cast<double2*>(out);
+    const bool split = parts > 1;
+    if (single) {
+      const float2* const p = static_cast<const float2*>(planes);
+      (split ? k_n2f_rows<float2, true> : k_n2f_rows<float2, false>)<<<grd, kN2fThreads, 0, st>>>(p, fx, n, nx, ny,
+                                                                                               cells, rows);
+    } else {
+      const double2* const p = static_cast<const double2*>(planes);
+      (split ? k_n2f_rows<double2, true> : k_n2f_rows<double2, false>)<<<grd, kN2fThreads, 0, st>>>(p, fx, n, nx, ny,
+                                                                                                 cells, rows);
+    }
+    (split ? k_n2f_finish<true> : k_n2f_finish<false>)<<<n, kN2fThreads, 0, st>>>(an, rows, parts, fy, ny, dx, k, r,
+                                                                                 total, o);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
