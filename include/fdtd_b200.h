@@ -135,7 +135,8 @@ extern "C" {
                                 interior march, then the split E pass */
 
 /* kernel kinds of fdtd_get_kernel_time */
-#define FDTD_TIME_STEP    0   /* the field-update kernel(s) of a step */
+#define FDTD_TIME_STEP    0   /* the field-update kernel(s) of a step, and the
+                                 phasors that run within a resident launch */
 #define FDTD_TIME_PHASOR  1   /* the phasor kernel of a step */
 
 /* Geometry and update constants of one simulation.

@@ -51,8 +51,8 @@
 // L2.
 //
 // Measured (float, us per step, single steps and pairs, phasors included):
-// 203 x 761 x 761 cells 1485 and 923; 101 x 381 x 381 243 and 184; double,
-// 101 x 381 x 381 650 and 322. At 203 x 761 x 761 the plain march takes 973 us
+// 203 x 761 x 761 cells 1485 and 930; 101 x 381 x 381 243 and 179 to 193 (by
+// where the fields lie); double, 101 x 381 x 381 650 and 320. At 203 x 761 x 761 the plain march takes 973 us
 // per pair (6.0 TB/s; 5.9 GB, of which 10 % is halo), the z faces 302, the
 // x ends 463, the y ends 123; those three are bound by instructions and
 // latency (IPC 1.3 to 1.5 at one block of 12 to 16 warps per SM), not by HBM.
