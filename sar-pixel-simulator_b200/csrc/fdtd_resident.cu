@@ -13,7 +13,9 @@
 // (after its predecessor's phasors), so that a launch ends on the set it began
 // with. A launch is of about two milliseconds (resident_launch_steps,
 // fdtd_capi.cu), because it holds every SM and stops every other stream; one
-// launch for the whole run is 0.2 % faster (one per millisecond 0.8 % slower).
+// launch for the whole run is 0.3 % to 0.8 % faster (31 x 39 x 39 cells 6.85
+// and 6.87 ms per 720 steps, 55 x 133 x 133 34.4 and 34.6 per 1200, 47 x 87 x 107
+// double 17.20 and 17.34 per 600), launches of four not measurably.
 // The updates are those of fdtd_vecn.cuh, equal bit for bit to the split
 // passes'; the phasor cell is the split step's (fdtd_split.cuh).
 //
